@@ -52,18 +52,50 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Q as a 2-D BF16 tensor [rows, cols], row-major; box = 64 columns x 128 rows, 128-byte swizzle.
+// Q as a 2-D BF16 tensor [rows, cols], row-major; box = 64 columns x 64 rows (a block's heads), 128-byte swizzle.
 cudaError_t make_q_map(CUtensorMap* map, const void* q, int64_t rows, int cols) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (fn == nullptr) return cudaErrorNotSupported;
     const cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
     const cuuint64_t strides[1] = {cuuint64_t(cols) * 2};
-    const cuuint32_t box[2] = {64, 128};
+    const cuuint32_t box[2] = {64, kHeadsPerBlock};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(q), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// Rows of 32-bit elements, `pitch` bytes apart, fetched four at a time by number (tile::gather4): box of `box_bytes`, one row high.
+cudaError_t make_row_map(CUtensorMap* map, const void* base, int64_t rows, int pitch, int box_bytes) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return cudaErrorNotSupported;
+    const cuuint64_t dims[2] = {cuuint64_t(pitch / 4), cuuint64_t(rows)};
+    const cuuint64_t strides[1] = {cuuint64_t(pitch)};
+    const cuuint32_t box[2] = {cuuint32_t(box_bytes / 4), 1};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// The record maps of the decode kernel (DecodeArgs): pool 0 the cache, pool 1 the window; an absent pool has none.
+template <int SRC>
+cudaError_t make_record_maps(DecodeArgs& a) {
+    cudaError_t e = cudaSuccess;
+    if constexpr (SRC == kSrcRefPaged) return e;               // fetched by untiled copies
+    const struct { const void* lat;  const void* rope;  int64_t rows; } pools[2] = {
+        {is_ref_layout(SRC) ? a.ref_kc : a.kv_pool, a.ref_kc_rope, is_ref_layout(SRC) ? int64_t(a.B) * a.ref_m_cur : int64_t(a.num_pages) * 64},
+        {is_ref_layout(SRC) ? a.ref_ks : a.win_pool, a.ref_ks_rope, is_ref_layout(SRC) ? int64_t(a.B) * a.ref_swa_len : int64_t(a.B) * a.win_cap}};
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+        if (pools[i].lat == nullptr || pools[i].rows <= 0) continue;
+        if (pools[i].rows > 0x7FFFFFFF) return cudaErrorInvalidValue;          // TMA coordinates are 32-bit
+        const int pitch = is_ref_layout(SRC) ? 448 : 656;
+        const int boxes[3] = {pitch, 256, is_ref_layout(SRC) ? 192 : 16};
+        for (int j = 0; j < 3 && e == cudaSuccess; ++j) e = make_row_map(&a.rec_map[i][j], pools[i].lat, pools[i].rows, pitch, boxes[j]);
+        if (e == cudaSuccess && is_ref_layout(SRC)) e = make_row_map(&a.rope_map[i], pools[i].rope, pools[i].rows, 128, 128);
+    }
+    return e;
 }
 
 bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -120,8 +152,10 @@ int64_t sched_slot_cap(int n_units, int num_splits, int num_pairs) {
 template <int NCHUNK, int SRC>
 cudaError_t launch_mma(DecodeArgs& a, int rows, const void* sched, cudaStream_t stream) {
     cudaError_t e = make_q_map(&a.q_map, a.q, int64_t(rows) * a.H, NCHUNK * 64);
+    if (e == cudaSuccess) e = make_record_maps<SRC>(a);
     if (e != cudaSuccess) return e;
-    a.wait_ns = g_wait_ns.load(std::memory_order_relaxed);
+    const unsigned long long wait_ns = g_wait_ns.load(std::memory_order_relaxed);
+    a.wait_ns = uint32_t(wait_ns < 4000000000ull ? wait_ns : 4000000000ull);
     a.dbg_drop_tile = g_drop_tile.load(std::memory_order_relaxed);
 #ifdef DSV4_TRACE
     a.trace = g_trace.load();
@@ -139,7 +173,7 @@ cudaError_t launch_mma(DecodeArgs& a, int rows, const void* sched, cudaStream_t 
         grid = dim3(2 * (pairs > 0 ? pairs : 1), 1, 1);
     }
     static std::atomic<bool> done[kMaxDevices];
-    constexpr int smem = SmemLayout<NCHUNK>::kTotal;
+    constexpr int smem = SmemLayout<NCHUNK, SRC>::kTotal;
     e = ensure_smem(decode_mma_kernel<NCHUNK, SRC>, smem, done);
     if (e != cudaSuccess) return e;
     decode_mma_kernel<NCHUNK, SRC><<<grid, kNumThreads, smem, stream>>>(a);

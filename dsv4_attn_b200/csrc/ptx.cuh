@@ -20,6 +20,13 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// Low half of the same clock: enough for limits of up to four seconds, and half the instructions.
+__device__ __forceinline__ uint32_t globaltimer_lo() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(t));
+    return t;
+}
+
 // ── mbarrier ────────────────────────────────────────────────────────────
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -38,31 +45,18 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+// How long a try_wait may suspend the warp before it reports failure: every retry takes a slot of the shared-memory port.
+constexpr uint32_t kSuspendNs = 1000;
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t"
         "}\n"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Non-blocking probe of a phase (try_wait may suspend the thread for a while).
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(kSuspendNs)
         : "memory");
     return ok != 0;
 }
@@ -80,6 +74,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_
             if (globaltimer_ns() - t0 > timeout_ns) return false;
         }
     }
+}
+
+// The same for a limit below four seconds and for a whole warp (all lanes get the same answer), with everything but the
+// first look out of line: kernels with many roles wait in many places, and code that does not fit the
+// instruction cache stalls all of them.
+__device__ __noinline__ bool mbar_wait_retry(uint32_t bar, uint32_t parity, uint32_t timeout_ns) {
+    const uint32_t t0 = globaltimer_lo();
+    bool done;
+    do { done = mbar_try_wait(bar, parity); } while (!done && globaltimer_lo() - t0 < timeout_ns);
+    return __all_sync(0xFFFFFFFFu, done);
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t timeout_ns) {
+    return __all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)) || mbar_wait_retry(bar, parity, timeout_ns);
 }
 
 // ── thread-block clusters / distributed shared memory ───────────────────
@@ -102,54 +109,11 @@ __device__ __forceinline__ uint32_t lds_cluster_u32(uint32_t caddr) {
 __device__ __forceinline__ void sts_cluster_u32(uint32_t caddr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(caddr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void sts_cluster_v4(uint32_t caddr, uint4 v) {
-    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(caddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-                 : "memory");
-}
-// Arrive on a barrier of another block of the cluster; this thread's earlier
-// stores to that block's shared memory are visible to whoever sees the arrival.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cbar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cbar) : "memory");
-}
-// Non-blocking probe of a local barrier whose arrivals may come from another block.
-__device__ __forceinline__ bool mbar_test_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait on a local barrier whose arrivals come from another block.
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint64_t timeout_ns) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    const uint64_t t0 = globaltimer_ns();
-    uint32_t polls = 0;
-    while (true) {
-        if (mbar_try_wait_cluster(bar, parity)) return true;
-        if ((++polls & 63u) == 0u) {
-            if (globaltimer_ns() - t0 > timeout_ns) return false;
-        }
-    }
+// Arrive on a barrier of another block of the cluster.  For hand-overs whose data stays in this block's own shared or
+// tensor memory, made visible there by a proxy or tcgen05 fence before: the arrival carries no data of its own, and a
+// release at cluster scope would also wait for every global load this thread has in flight (measured: 1.2 us a time).
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cbar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cbar) : "memory");
 }
 
 // ── fences ──────────────────────────────────────────────────────────────
@@ -205,18 +169,10 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
-// The same store with the 32 words given as eight 16-byte vectors.
-__device__ __forceinline__ void tmem_st32_v4(uint32_t taddr, const uint4* v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        :
-        : "r"(taddr), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
-          "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w),
-          "r"(v[4].x), "r"(v[4].y), "r"(v[4].z), "r"(v[4].w), "r"(v[5].x), "r"(v[5].y), "r"(v[5].z), "r"(v[5].w),
-          "r"(v[6].x), "r"(v[6].y), "r"(v[6].z), "r"(v[6].w), "r"(v[7].x), "r"(v[7].y), "r"(v[7].z), "r"(v[7].w)
-        : "memory");
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4& a, const uint4& b) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(a.x), "r"(a.y),
+                 "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -266,38 +222,20 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, bool a_mn_ma
            | (static_cast<uint32_t>(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void mma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+// One lane of a converged warp, the same one every time.  The branch an issuing warp takes on it is known to be
+// warp-uniform, so that operands of tcgen05 instructions can live in uniform registers: measured, a stream of
+// M = 128, N = 64 MMAs issues at one per 13 cycles behind this and at one per 45 behind `if (lane == 0)`.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand (128 rows x 16 BF16 per K step)
-// is read from tensor memory, lane = row, two K-consecutive BF16 per 32-bit column.
-__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// Variants that take the operand descriptors as (low, high) 32-bit halves.
-__device__ __forceinline__ void mma_bf16_ss2(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
-                                             uint32_t idesc, uint32_t accumulate) {
+// ── MMA over a cluster pair (cta_group::2), issued by one thread of the even block ──
+// M = 128: each block supplies 64 rows of A and half of the N rows (columns) of B, at the same shared-memory
+// address in both, and receives its 64 rows of D: tensor-memory lanes 0-63 hold columns [0, N/2), lanes 64-127
+// columns [N/2, N) of the same rows.
+__device__ __forceinline__ void mma2_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
@@ -305,37 +243,64 @@ __device__ __forceinline__ void mma_bf16_ss2(uint32_t d_tmem, uint32_t a_lo, uin
         "mov.b64 da, {%1, %3};\n\t"
         "mov.b64 db, {%2, %3};\n\t"
         "setp.ne.b32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t"
         "}\n"
         :
         : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void mma_bf16_ts2(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi,
-                                             uint32_t idesc, uint32_t accumulate) {
+// The same with A in tensor memory: 64 rows per block, in lanes 0-63 and again in lanes 64-127, two 16-bit values per column.
+__device__ __forceinline__ void mma2_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
         ".reg .b64 db;\n\t"
         "mov.b64 db, {%2, %3};\n\t"
         "setp.ne.b32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %4, p;\n\t"
         "}\n"
         :
         : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// Arrive once on the barrier at this offset in both blocks of the pair when every MMA this thread issued so far has finished.
+__device__ __forceinline__ void mma2_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(uint16_t(3))
+                 : "memory");
+}
+// Both blocks of the pair take part in allocating and freeing.
+__device__ __forceinline__ void tmem2_alloc(uint32_t dst, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem2_relinquish() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem2_dealloc(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// Rendezvous of `threads` threads on named barrier `id`; true if any of them passed a true predicate.
+__device__ __forceinline__ bool bar_any(uint32_t id, uint32_t threads, bool pred) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "barrier.red.or.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"(id), "r"(threads), "r"(uint32_t(pred))
+        : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void bar_sync(uint32_t id, uint32_t threads) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 // Arrive once on `bar` when every MMA this thread issued so far has finished.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
-}
-
-// The same for a barrier given by its cluster-wide address (mapa): it may live in the other
-// block of a cluster pair.
-__device__ __forceinline__ void mma_commit_cluster(uint32_t cbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cbar) : "memory");
 }
 
 // ── TMA ─────────────────────────────────────────────────────────────────
@@ -350,11 +315,51 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const void* tenso
         : "memory");
 }
 
+// Four rows of a row-major tensor named by their numbers (tile::gather4; the map's box is one row high), laid down one
+// after the other at smem_dst, which is a multiple of 128 bytes.
+__device__ __forceinline__ void tma_gather4(uint32_t smem_dst, const void* tensor_map, int x, const int4& rows, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        :
+        : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tensor_map)), "r"(x), "r"(rows.x), "r"(rows.y), "r"(rows.z), "r"(rows.w), "r"(bar)
+        : "memory");
+}
+// Untiled copy; both addresses and the size are multiples of 16 bytes.
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :
+                 : "r"(smem_dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
 // ── small math / memory helpers ─────────────────────────────────────────
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Two FP32 operations in one instruction.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
 __device__ __forceinline__ uint4 ldg_nc_v4(const void* p) {
@@ -383,6 +388,25 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t saddr) {
     return v;
 }
 
+__device__ __forceinline__ uint32_t lds_u32(uint32_t saddr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 lds_v2(uint32_t saddr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(saddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t lds_u8(uint32_t saddr) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_v2(uint32_t saddr, uint2 v) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(saddr), "r"(v.x), "r"(v.y) : "memory");
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -397,13 +421,6 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
 // two BF16 in one word -> the same two values as FP16 (exact for magnitudes in FP16's normal range)
 __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
     return pack_f16x2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-}
-
-// two FP8 e4m3 in the low 16 bits -> two FP16 (exact), element order kept
-__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two_bytes) {
-    uint32_t r;
-    asm("{\n\t.reg .b16 t;\n\tcvt.u16.u32 t, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, t;\n\t}" : "=r"(r) : "r"(two_bytes));
-    return r;
 }
 
 // four FP8 e4m3 in one word -> four FP16 (exact), element order kept: lo = elements 0, 1; hi = elements 2, 3
