@@ -15,10 +15,12 @@ __all__ = ["LIB", "library_path", "layout", "synth", *_API]
 
 
 def __getattr__(name):
+    # (what is found is kept as an attribute of the package: this function costs a microsecond, and a caller looks its
+    # operators up on every call)
     if name in _API:
-        return getattr(importlib.import_module(".api", __name__), name)
+        return globals().setdefault(name, getattr(importlib.import_module(".api", __name__), name))
     if name in ("LIB", "library_path"):
-        return getattr(importlib.import_module("._lib", __name__), name)
+        return globals().setdefault(name, getattr(importlib.import_module("._lib", __name__), name))
     if name in ("layout", "synth", "api", "build"):
         return importlib.import_module("." + name, __name__)
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")

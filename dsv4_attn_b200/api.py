@@ -5,7 +5,12 @@ Each function follows the pattern of the reference's operator boundary
 a plain parameter struct with raw device pointers, launch on the current
 CUDA stream, return tensors the callee allocated (unless the caller passes
 them).  The arithmetic is done by libdsv4_attn.so only; nothing here computes
-on the host and nothing falls back to PyTorch ops."""
+on the host and nothing falls back to PyTorch ops.
+
+Each function first hands its arguments to the extension module `_host`, which
+does all of that in native code (3 to 6 us a call, where the Python below takes
+15 to 35) and answers None when an argument is not the ordinary case; the checks below
+then say what is wrong, or serve the rarer forms."""
 from __future__ import annotations
 
 import ctypes as C
@@ -13,7 +18,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 from .layout import D_QK, D_LATENT, ENTRY_BYTES, PAGE_ENTRIES
 
 MAX_SPLITS = 64
@@ -48,6 +53,12 @@ def _stream(device) -> C.c_void_p:
 def _rc(rc: int, what: str) -> None:
     if rc != 0:
         raise Dsv4Error(f"{what} failed: cudaError={rc}")
+
+
+_host.bind(*(C.cast(getattr(_lib.LIB, name), C.c_void_p).value for name in (
+    "dsv4_csa_sparse_decode_fwd", "dsv4_hca_dense_decode_fwd", "dsv4_hca_packed_decode_fwd", "hca_decode_fwd", "dsv4_rope_norm_fwd",
+    "dsv4_kv_quantize_insert", "dsv4_csa_compress_reduce_fwd", "dsv4_hca_compress_fwd", "dsv4_indexer_topk_fwd", "dsv4_attn_combine",
+    "dsv4_attn_plan", "dsv4_attn_plan_splits")))
 
 
 def plan_splits(rows: int, H: int, max_len: int, num_sms: int = 0) -> int:
@@ -89,9 +100,15 @@ class Plan:
         self.partial_o = torch.empty(max(po.value // 4, 4), dtype=torch.float32, device=device)
         self.partial_lse = torch.empty(max(pl.value // 4, 4), dtype=torch.float32, device=device)
         self.lengths = lengths
+        # what the decode calls and remake() take of a plan
+        self.fast = (kind, B, s_q, H, topk, self.sched, self.partial_o, self.partial_lse)
+        self._request = (kind, B, s_q, H, topk, num_splits, num_sms, *lengths, self.sched)
         self.remake()
 
     def remake(self):
+        rc = _host.plan(*self._request)
+        if rc == 0:
+            return self
         topk_len, kv_len, win_len = self.lengths
         p = _lib.PlanParams(kind=self.kind, B=self.B, s_q=self.s_q, H=self.H, topk=self.topk, num_splits=self.num_splits,
                             num_sms=self.num_sms, topk_len=_ptr(topk_len), kv_len=_ptr(kv_len), win_len=_ptr(win_len),
@@ -187,6 +204,11 @@ def csa_sparse_decode(q, kv_pool, block_table, indices, sm_scale, *, kv_len=None
     kv_len optional int32 [B, s_q]; topk_len optional int32 [B, s_q] (only the
     first topk_len slots of each list are read).  Returns (out bf16 [B, s_q, H, 512],
     lse f32 [B, s_q, H])."""
+    if impl == "mma" and not check_fp16_range:
+        r = _host.csa(q, kv_pool, block_table, indices, sm_scale, kv_len, topk_len, attn_sink, num_splits, out, lse, workspace, status,
+                      None if plan is None else plan.fast)
+        if r is not None:
+            return r if type(r) is tuple else _rc(r, "dsv4_csa_sparse_decode")
     _cuda_contig(indices, "indices", torch.int32, 3)
     topk = indices.shape[-1]
     if impl == "simt":
@@ -253,6 +275,11 @@ def hca_dense_decode(q, kv_pool, block_table, kv_len, win_pool, win_len, sm_scal
     [B, W, 656].  `max_len` (longest kv_len + win_len) only steers the split
     planner; when omitted the block-table capacity is used so that no device
     read-back is needed."""
+    if impl == "mma" and not check_fp16_range:
+        r = _host.hca(q, kv_pool, block_table, kv_len, win_pool, win_len, sm_scale, attn_sink, num_splits, out, lse, workspace, status, max_len,
+                      None if plan is None else plan.fast)
+        if r is not None:
+            return r if type(r) is tuple else _rc(r, "dsv4_hca_dense_decode")
     _cuda_contig(kv_len, "kv_len", torch.int32, 2)
     _cuda_contig(win_len, "win_len", torch.int32, 2)
     _cuda_contig(win_pool, "win_pool", torch.uint8, 3)
@@ -284,6 +311,9 @@ def hca_dense_decode(q, kv_pool, block_table, kv_len, win_pool, win_len, sm_scal
 def combine(partial_o, partial_lse, *, attn_sink=None, out=None, lse=None):
     """Merge split partials: partial_o f32 [S, N, H, 512], partial_lse f32
     [S, N, H] (log2).  Returns (out bf16 [N, H, 512], lse f32 [N, H])."""
+    r = _host.combine(partial_o, partial_lse, attn_sink, out, lse)
+    if r is not None:
+        return r if type(r) is tuple else _rc(r, "dsv4_attn_combine")
     _cuda_contig(partial_o, "partial_o", torch.float32, 4)
     _cuda_contig(partial_lse, "partial_lse", torch.float32, 3)
     S, N, H, D = partial_o.shape
@@ -309,6 +339,9 @@ def hca_decode_fwd(Q, Kc, Kc_s, Kc_rope, Kswa, Kswa_s, Kswa_rope, sink_logits, s
     """The reference's entry point on its own cache layout (448 e4m3 + 7 UE8M0
     + 64 bf16 per entry), same arguments as the reference's ctypes launcher
     (bench/bench/candidates/hca_custom_decode.py:124-158)."""
+    r = _host.planes(Q, Kc, Kc_s, Kc_rope, Kswa, Kswa_s, Kswa_rope, sink_logits, sm_scale, M_cur, swa_len, O, partial_O, partial_lse)
+    if r is not None:
+        return _rc(r, "hca_decode_fwd") if type(r) is int else r
     _cuda_contig(Q, "Q", torch.bfloat16, 3)
     B, n_h, dq = Q.shape
     c = Kc.shape[-1]
@@ -333,6 +366,9 @@ def csa_compress_reduce_fwd(C_a, C_b, Z_a, Z_b, B_a, B_b, m, *, out=None):
     reference's csa_compress_reduce_fwd (csa/interface.h:21-85, bound in
     csa/pybind.cpp:5-17): four BF16 streams [B, n, c_out], two BF16 biases
     [m, c_out], returns BF16 [B, n/m, c_out] allocated here."""
+    r = _host.csa_compress(C_a, C_b, Z_a, Z_b, B_a, B_b, m, out)
+    if r is not None:
+        return _rc(r, "dsv4_csa_compress_reduce_fwd") if type(r) is int else r
     for name, t in (("C_a", C_a), ("C_b", C_b), ("Z_a", Z_a), ("Z_b", Z_b)):
         _check(t.is_cuda, "all inputs must be on cuda")
         _check(t.dtype == torch.bfloat16, f"{name} must be bf16")
@@ -376,6 +412,9 @@ def hca_compress_fwd(C_, Z, bias, m, *, out=None, kv_pool=None, block_table=None
     With kv_pool / block_table / insert_pos (c == 576) the rows are also quantised and
     written into the paged cache as entries insert_pos[b] + i; `want_out=False` skips the
     dense output then."""
+    r = _host.hca_compress(C_, Z, bias, m, out, kv_pool, block_table, insert_pos, status, want_out)
+    if r is not None:
+        return None if r is False else (_rc(r, "dsv4_hca_compress_fwd") if type(r) is int else r)
     for name, t in (("C", C_), ("Z", Z)):
         _cuda_contig(t, name, torch.bfloat16, 3)
     _check(C_.shape == Z.shape, "C and Z must be equal-shaped [B, n, c]")
@@ -403,6 +442,9 @@ def hca_compress_fwd(C_, Z, bias, m, *, out=None, kv_pool=None, block_table=None
 def kv_quantize_insert(rows, kv_pool, block_table, insert_pos, *, n_rows=None, status=None) -> None:
     """Quantise BF16 rows [B, T, 576] into 656-byte cache entries and write them at logical
     positions insert_pos[b] + t of request b (in place, into kv_pool)."""
+    r = _host.insert(rows, kv_pool, block_table, insert_pos, n_rows, status)
+    if r is not None:
+        return None if r is True else _rc(r, "dsv4_kv_quantize_insert")
     _cuda_contig(rows, "rows", torch.bfloat16, 3)
     B, T, c = rows.shape
     _check(c == D_QK, f"rows must be [B, T, {D_QK}]")
@@ -425,6 +467,10 @@ def hca_packed_decode(q, kv_pages, block_table, m_cur, swa_pages, swa_block_tabl
     Dsv4HcaPackedDecodeParams in include/dsv4_attn.h), per-request lengths m_cur / swa_len
     int32 [B].  q bf16 [B, H, 512]; pools uint8 [pages, page_size*584].  Returns
     (out bf16 [B, H, 512], lse f32 [B, H])."""
+    r = _host.packed(q, kv_pages, block_table, m_cur, swa_pages, swa_block_table, swa_len, sm_scale, page_size, attn_sink, num_splits, out, lse,
+                     workspace, status)
+    if r is not None:
+        return r if type(r) is tuple else _rc(r, "dsv4_hca_packed_decode_fwd")
     _cuda_contig(q, "q", torch.bfloat16, 3)
     B, H, dq = q.shape
     _check(dq == 512, "q must be [B, H, 512]")
@@ -472,6 +518,9 @@ def rope_norm(x, positions, *, norm_weight=None, eps=1e-6, n_rope=64, theta=1000
     reference's apply_rope followed by rms_norm, bench/bench/reference.py:35-70, 281-287).
     `inverse=True` rotates by -position (the inverse RoPE on the attention output,
     reference.py:308-309).  `out` may be x itself."""
+    r = _host.rope_norm(x, positions, norm_weight, eps, n_rope, theta, inverse, out)
+    if r is not None:
+        return _rc(r, "dsv4_rope_norm_fwd") if type(r) is int else r
     _cuda_contig(x, "x", torch.bfloat16, 3)
     rows, vecs, c = x.shape
     _cuda_contig(positions, "positions", torch.int32, 1)
@@ -500,6 +549,9 @@ def indexer_topk(q_fp8, q_weight, key_pages, block_table, n_vis, k, *, scores=No
     Dsv4IndexerTopkParams).  q_fp8 uint8 [B, s_q, 64, 128] (e4m3), q_weight f32 [B, s_q, 64],
     key_pages uint8 [pages, 8448], block_table int32 [B, max_pages], n_vis int32 [B, s_q].
     Returns (indices int32 [B, s_q, k], scores f32 [B*s_q, stride])."""
+    r = _host.indexer(q_fp8, q_weight, key_pages, block_table, n_vis, k, scores, out, status)
+    if r is not None:
+        return r if type(r) is tuple else _rc(r, "dsv4_indexer_topk_fwd")
     _cuda_contig(q_fp8, "q_fp8", torch.uint8, 4)
     B, s_q, nh, dim = q_fp8.shape
     _check(nh == INDEXER_HEADS and dim == INDEXER_DIM, "q_fp8 must be [B, s_q, 64, 128]")

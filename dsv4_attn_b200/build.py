@@ -1,10 +1,11 @@
 #!/usr/bin/env python3
-"""Build libdsv4_attn.so in-tree with plain nvcc (no torch, no pybind needed).
+"""Build the two shared objects in-tree: libdsv4_attn.so (the kernels behind their C ABI; plain nvcc, no torch) and
+_host.so (the Python operator surface's fast path; g++ against torch's headers).
 
-    python -m dsv4_attn_b200.build            # builds dsv4_attn_b200/libdsv4_attn.so
+    python -m dsv4_attn_b200.build            # builds what is out of date
     python -m dsv4_attn_b200.build --ptxas-v  # also prints registers / spills / shared memory
 
-The recipe mirrors the reference project's standalone build
+The recipe of the first mirrors the reference project's standalone build
 (hca/compile.py:68-83): one nvcc call, sm_100a only, a shared object that is
 loaded with ctypes.
 """
@@ -20,17 +21,40 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 SOURCE = HERE / "csrc" / "api.cu"
 OUT = HERE / "libdsv4_attn.so"
-DEPS = sorted((HERE / "csrc").glob("*")) + [HERE.parent / "include" / "dsv4_attn.h"]
+HEADER = HERE.parent / "include" / "dsv4_attn.h"
+HOST_SOURCE = HERE / "csrc" / "host.cpp"
+HOST_OUT = HERE / "_host.so"
+DEPS = [p for p in sorted((HERE / "csrc").glob("*")) if p != HOST_SOURCE] + [HEADER]
 
 
-def needs_build() -> bool:
-    if not OUT.exists():
+def needs_build(out: Path = OUT, deps=tuple(DEPS)) -> bool:
+    if not out.exists():
         return True
-    t = OUT.stat().st_mtime
-    return any(p.stat().st_mtime > t for p in DEPS)
+    t = out.stat().st_mtime
+    return any(p.stat().st_mtime > t for p in deps)
+
+
+def build_host(force: bool = False, quiet: bool = False) -> Path:
+    if not force and not needs_build(HOST_OUT, (HOST_SOURCE, HEADER)):
+        return HOST_OUT
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    nvcc = shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc"
+    cuda = Path(nvcc).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{sysconfig.get_paths()['include']}", "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+           "-isystem", str(cuda / "include"), "-o", str(HOST_OUT), str(HOST_SOURCE), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch", "-ltorch_python"]
+    if not quiet:
+        print(" ".join(cmd), flush=True)
+    subprocess.run(cmd, check=True)
+    return HOST_OUT
 
 
 def build(force: bool = False, ptxas_v: bool = False, quiet: bool = False) -> Path:
+    build_host(force=force and not ptxas_v, quiet=quiet)
     if not force and not needs_build():
         return OUT
     nvcc = shutil.which(os.environ.get("NVCC", "nvcc")) or "/usr/local/cuda/bin/nvcc"

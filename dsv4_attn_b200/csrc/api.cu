@@ -79,23 +79,53 @@ cudaError_t make_row_map(CUtensorMap* map, const void* base, int64_t rows, int p
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// The record maps of the decode kernel (DecodeArgs): pool 0 the cache, pool 1 the window; an absent pool has none.
+// The record maps of one pool (DecodeArgs::rec_map, rope_map).  A map is a function of the pool's address, rows and kind alone, and a
+// program's pools stay where they are from call to call, so each thread keeps the last few it made (2 us a call otherwise).
+struct PoolMaps {
+    const void* lat = nullptr;
+    const void* rope = nullptr;
+    int64_t rows = 0;
+    bool ref = false;
+    CUtensorMap rec[3], rope_map;
+};
+cudaError_t pool_maps(const PoolMaps** out, const void* lat, const void* rope, int64_t rows, bool ref) {
+    constexpr int kKept = 8;
+    static thread_local PoolMaps kept[kKept];
+    static thread_local int next = 0;
+    for (const PoolMaps& m : kept)
+        if (m.lat == lat && m.rope == rope && m.rows == rows && m.ref == ref) { *out = &m;  return cudaSuccess; }
+    if (rows > 0x7FFFFFFF) return cudaErrorInvalidValue;                   // TMA coordinates are 32-bit
+    PoolMaps& m = kept[next];
+    m.lat = nullptr;
+    const int pitch = ref ? 448 : 656;
+    const int boxes[3] = {pitch, 256, ref ? 192 : 16};
+    cudaError_t e = cudaSuccess;
+    for (int j = 0; j < 3 && e == cudaSuccess; ++j) e = make_row_map(&m.rec[j], lat, rows, pitch, boxes[j]);
+    if (e == cudaSuccess && ref) e = make_row_map(&m.rope_map, rope, rows, 128, 128);
+    if (e != cudaSuccess) return e;
+    m.lat = lat;  m.rope = rope;  m.rows = rows;  m.ref = ref;
+    next = (next + 1) % kKept;
+    *out = &m;
+    return e;
+}
+
+// The record maps of a decode call: pool 0 the cache, pool 1 the window; an absent pool has none.
 template <int SRC>
 cudaError_t make_record_maps(DecodeArgs& a) {
-    cudaError_t e = cudaSuccess;
-    if constexpr (SRC == kSrcRefPaged) return e;               // fetched by untiled copies
+    if constexpr (SRC == kSrcRefPaged) return cudaSuccess;                 // fetched by untiled copies
+    constexpr bool ref = is_ref_layout(SRC);
     const struct { const void* lat;  const void* rope;  int64_t rows; } pools[2] = {
-        {is_ref_layout(SRC) ? a.ref_kc : a.kv_pool, a.ref_kc_rope, is_ref_layout(SRC) ? int64_t(a.B) * a.ref_m_cur : int64_t(a.num_pages) * 64},
-        {is_ref_layout(SRC) ? a.ref_ks : a.win_pool, a.ref_ks_rope, is_ref_layout(SRC) ? int64_t(a.B) * a.ref_swa_len : int64_t(a.B) * a.win_cap}};
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+        {ref ? a.ref_kc : a.kv_pool, a.ref_kc_rope, ref ? int64_t(a.B) * a.ref_m_cur : int64_t(a.num_pages) * 64},
+        {ref ? a.ref_ks : a.win_pool, a.ref_ks_rope, ref ? int64_t(a.B) * a.ref_swa_len : int64_t(a.B) * a.win_cap}};
+    for (int i = 0; i < 2; ++i) {
         if (pools[i].lat == nullptr || pools[i].rows <= 0) continue;
-        if (pools[i].rows > 0x7FFFFFFF) return cudaErrorInvalidValue;          // TMA coordinates are 32-bit
-        const int pitch = is_ref_layout(SRC) ? 448 : 656;
-        const int boxes[3] = {pitch, 256, is_ref_layout(SRC) ? 192 : 16};
-        for (int j = 0; j < 3 && e == cudaSuccess; ++j) e = make_row_map(&a.rec_map[i][j], pools[i].lat, pools[i].rows, pitch, boxes[j]);
-        if (e == cudaSuccess && is_ref_layout(SRC)) e = make_row_map(&a.rope_map[i], pools[i].rope, pools[i].rows, 128, 128);
+        const PoolMaps* m = nullptr;
+        const cudaError_t e = pool_maps(&m, pools[i].lat, pools[i].rope, pools[i].rows, ref);
+        if (e != cudaSuccess) return e;
+        for (int j = 0; j < 3; ++j) a.rec_map[i][j] = m->rec[j];
+        if (ref) a.rope_map[i] = m->rope_map;
     }
-    return e;
+    return cudaSuccess;
 }
 
 bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -116,9 +146,14 @@ cudaError_t ensure_smem(Kernel kernel, int bytes, std::atomic<bool>* done_per_de
     return cudaSuccess;
 }
 
+// SMs of the current device (asked for once per device).
 int device_sms() {
+    static std::atomic<int> known[kMaxDevices];
     int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return sms;
+    const int k = known[dev].load(std::memory_order_relaxed);
+    if (k > 0) return k;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) known[dev].store(sms, std::memory_order_relaxed);
     return sms;
 }
 
@@ -529,9 +564,9 @@ extern "C" int dsv4_attn_plan_splits(int rows, int H, int max_len, int num_sms) 
     if (rows <= 0 || H <= 0 || max_len < 0) return -int(cudaErrorInvalidValue);
     if (num_sms <= 0) {
         int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+        const cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return -int(e);
+        num_sms = device_sms();
     }
     const int tiles = (max_len + kTileN - 1) / kTileN;
     if (tiles <= 1) return 1;
@@ -636,8 +671,7 @@ extern "C" int dsv4_csa_compress_reduce_fwd(const Dsv4CsaCompressReduceParams* p
                      (p->stride_out_b % 8 == 0) && (p->stride_out_blk % 8 == 0) && aligned(p->C_a, 16) &&
                      aligned(p->C_b, 16) && aligned(p->Z_a, 16) && aligned(p->Z_b, 16) && aligned(p->B_a, 16) &&
                      aligned(p->B_b, 16) && aligned(p->out, 16);
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const int64_t items = int64_t(a.B) * a.n_blocks * (vec ? a.c_out / 4 : a.c_out);
     const int64_t want = (items + kCompressThreads - 1) / kCompressThreads;
     // at most 8 blocks per SM (two waves of the 4 resident ones); beyond that the grid-stride loop takes over
@@ -699,8 +733,7 @@ extern "C" int dsv4_kv_quantize_insert(const Dsv4KvQuantizeInsertParams* p, void
     a.stride_b = p->stride_b;  a.stride_t = p->stride_t;
     a.n_rows = p->n_rows;
     if (!fill_cache_dest(p->dst, p->B, a.dst)) return int(cudaErrorInvalidValue);
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const int64_t rows = int64_t(a.B) * a.T;
     const int64_t want = (rows + kInsertThreads / 32 - 1) / (kInsertThreads / 32);
     const int64_t cap = int64_t(sms) * 8;
@@ -770,8 +803,7 @@ extern "C" int dsv4_rope_norm_fwd(const Dsv4RopeNormParams* p, void* stream) {
     a.out = static_cast<__nv_bfloat16*>(p->out);
     a.positions = p->positions;
     a.weight = static_cast<const __nv_bfloat16*>(p->norm_weight);
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const int64_t items = a.n_rows * ((a.vecs_per_row + kRopeGroup - 1) / kRopeGroup);
     const int64_t want = (items + kRopeNormThreads / 32 - 1) / (kRopeNormThreads / 32);
     const int64_t cap = int64_t(sms) * 8;
@@ -809,8 +841,7 @@ extern "C" int dsv4_indexer_topk_fwd(const Dsv4IndexerTopkParams* p, void* strea
     if (e == cudaSuccess) e = make_byte_map(&a.scale_map, p->key_pages, uint64_t(p->num_pages) * kIdxPageRows, 2, false);
     if (e == cudaSuccess) e = make_byte_map(&a.q_map, p->q_fp8, uint64_t(p->B) * p->s_q * kIdxHeads, uint32_t(p->s_q * kIdxHeads), true);
     if (e != cudaSuccess) return int(e);
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const int tiles_cap = (p->max_pages + 1) / 2;
     // Blocks per request: two blocks are resident per SM; the time is (waves of resident blocks) x
     // (tiles per block + a fixed set-up of about two tiles).  Pick the count that minimises it.
