@@ -184,6 +184,25 @@ int64_t sched_slot_cap(int n_units, int num_splits, int num_pairs) {
     return num_splits > 1 ? int64_t(n_units) * num_splits : 2 * int64_t(num_pairs);
 }
 
+// Every kernel of the library is launched as a programmatic dependent of whatever precedes it in the stream (the kernels
+// wait before they touch memory, see ptx.cuh): in a chain of small kernels the launch and set-up of each - 2 to 3 us when a
+// kernel takes 4 to 10 - then lie under the tail of the one before.  A preceding kernel that never triggers makes it an
+// ordinary launch.
+template <class Args>
+cudaError_t launch(void (*kernel)(Args), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args& args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = (g_dbg.load(std::memory_order_relaxed) & 64) ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
 template <int NCHUNK, int SRC>
 cudaError_t launch_mma(DecodeArgs& a, int rows, const void* sched, cudaStream_t stream) {
     cudaError_t e = make_q_map(&a.q_map, a.q, int64_t(rows) * a.H, NCHUNK * 64);
@@ -211,8 +230,7 @@ cudaError_t launch_mma(DecodeArgs& a, int rows, const void* sched, cudaStream_t 
     constexpr int smem = SmemLayout<NCHUNK, SRC>::kTotal;
     e = ensure_smem(decode_mma_kernel<NCHUNK, SRC>, smem, done);
     if (e != cudaSuccess) return e;
-    decode_mma_kernel<NCHUNK, SRC><<<grid, kNumThreads, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch(decode_mma_kernel<NCHUNK, SRC>, grid, kNumThreads, smem, stream, a);
 }
 
 template <int SRC>
@@ -227,27 +245,9 @@ cudaError_t launch_simt(const DecodeArgs& a, int rows, int max_tok, cudaStream_t
     return cudaGetLastError();
 }
 
-// after_decode: the launch directly follows this library's decode launch on the same stream; the merge is then
-// launched as its programmatic dependent, so that its blocks are resident (and waiting) when the last decode
-// blocks are in their epilogue.
-cudaError_t launch_combine(const CombineArgs& c, cudaStream_t stream, bool after_decode = false) {
+cudaError_t launch_combine(const CombineArgs& c, cudaStream_t stream) {
     const int64_t units = int64_t(c.N) * c.H;
-    const int blocks = int((units + kCombineWarps - 1) / kCombineWarps);
-    if (after_decode && !(g_dbg.load(std::memory_order_relaxed) & 64)) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(kCombineWarps * 32);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, combine_kernel, c);
-    }
-    combine_kernel<<<blocks, kCombineWarps * 32, 0, stream>>>(c);
-    return cudaGetLastError();
+    return launch(combine_kernel, dim3(unsigned((units + kCombineWarps - 1) / kCombineWarps)), kCombineWarps * 32, 0, stream, c);
 }
 
 CombineArgs contiguous_combine(int rows, int H, int S, const float* po, const float* pl, void* out, float* lse,
@@ -368,11 +368,11 @@ int decode_fwd(DecodeArgs& a, const void* sched, cudaStream_t stream) {
         c.unit_nsplits = static_cast<const int32_t*>(sched) + l.unit_nsplits;
         c.unit_slot = static_cast<const int32_t*>(sched) + l.unit_slot;
         c.hgs = hgs;
-        e = launch_combine(c, stream, true);
+        e = launch_combine(c, stream);
     } else if (a.num_splits > 1) {
         CombineArgs c = contiguous_combine(rows, a.H, a.num_splits, a.partial_o, a.partial_lse, a.out, a.lse, a.attn_sink,
                                            true);
-        e = launch_combine(c, stream, true);
+        e = launch_combine(c, stream);
     }
     return e == cudaSuccess ? 0 : launch_failed(e);
 }
@@ -466,8 +466,7 @@ extern "C" int dsv4_attn_plan(const Dsv4PlanParams* p, void* stream) {
     if (p != nullptr && p->num_sms > device_sms()) { t_last_error = "num_sms exceeds the device";  return int(cudaErrorInvalidValue); }
     const int rc = fill_plan(p, p ? static_cast<int32_t*>(p->sched) : nullptr, a);
     if (rc != 0) return rc;
-    plan_kernel<<<1, kPlanThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch(plan_kernel, dim3(1), kPlanThreads, 0, static_cast<cudaStream_t>(stream), a);
     return e == cudaSuccess ? 0 : launch_failed(e);
 }
 
@@ -646,7 +645,7 @@ extern "C" int hca_decode_fwd(const void* Q,
     if (e != cudaSuccess) return int(e);
     if (splits > 1) {
         CombineArgs cb = contiguous_combine(B, n_h, splits, a.partial_o, a.partial_lse, O, nullptr, a.attn_sink, true);
-        e = launch_combine(cb, s, true);
+        e = launch_combine(cb, s);
     }
     return int(e);
 }
@@ -677,10 +676,8 @@ extern "C" int dsv4_csa_compress_reduce_fwd(const Dsv4CsaCompressReduceParams* p
     // at most 8 blocks per SM (two waves of the 4 resident ones); beyond that the grid-stride loop takes over
     const int64_t cap = int64_t(sms) * 8;
     const int blocks = int(want < cap ? (want > 0 ? want : 1) : cap);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (vec) compress_reduce_kernel<4, 4><<<blocks, kCompressThreads, 0, s>>>(a);
-    else compress_reduce_kernel<4, 1><<<blocks, kCompressThreads, 0, s>>>(a);
-    return int(cudaGetLastError());
+    return int(launch(vec ? compress_reduce_kernel<4, 4> : compress_reduce_kernel<4, 1>, dim3(blocks), kCompressThreads, 0,
+                      static_cast<cudaStream_t>(stream), a));
 }
 
 
@@ -720,8 +717,7 @@ extern "C" int dsv4_hca_compress_fwd(const Dsv4HcaCompressParams* p, void* strea
     if (rows_out > 0x7FFFFFFF) return int(cudaErrorInvalidValue);
     const dim3 grid(unsigned(rows_out), unsigned((a.c / 8 + kHcaVecsPerBlock - 1) / kHcaVecsPerBlock), 1);
     if (grid.y > 65535u) return int(cudaErrorInvalidValue);
-    hca_compress_kernel<<<grid, kHcaCompressThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    return int(cudaGetLastError());
+    return int(launch(hca_compress_kernel, grid, kHcaCompressThreads, 0, static_cast<cudaStream_t>(stream), a));
 }
 
 extern "C" int dsv4_kv_quantize_insert(const Dsv4KvQuantizeInsertParams* p, void* stream) {
@@ -738,8 +734,7 @@ extern "C" int dsv4_kv_quantize_insert(const Dsv4KvQuantizeInsertParams* p, void
     const int64_t want = (rows + kInsertThreads / 32 - 1) / (kInsertThreads / 32);
     const int64_t cap = int64_t(sms) * 8;
     const int blocks = int(want < cap ? want : cap);
-    kv_quantize_insert_kernel<<<blocks, kInsertThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    return int(cudaGetLastError());
+    return int(launch(kv_quantize_insert_kernel, dim3(blocks), kInsertThreads, 0, static_cast<cudaStream_t>(stream), a));
 }
 
 
@@ -784,7 +779,7 @@ extern "C" int dsv4_hca_packed_decode_fwd(const Dsv4HcaPackedDecodeParams* p, vo
     if (a.num_splits > 1) {
         CombineArgs cb = contiguous_combine(p->B, p->H, a.num_splits, a.partial_o, a.partial_lse, a.out, a.lse, a.attn_sink,
                                             true);
-        e = launch_combine(cb, s, true);
+        e = launch_combine(cb, s);
     }
     return int(e);
 }
@@ -807,8 +802,7 @@ extern "C" int dsv4_rope_norm_fwd(const Dsv4RopeNormParams* p, void* stream) {
     const int64_t items = a.n_rows * ((a.vecs_per_row + kRopeGroup - 1) / kRopeGroup);
     const int64_t want = (items + kRopeNormThreads / 32 - 1) / (kRopeNormThreads / 32);
     const int64_t cap = int64_t(sms) * 8;
-    rope_norm_kernel<<<int(want < cap ? want : cap), kRopeNormThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    return int(cudaGetLastError());
+    return int(launch(rope_norm_kernel, dim3(unsigned(want < cap ? want : cap)), kRopeNormThreads, 0, static_cast<cudaStream_t>(stream), a));
 }
 
 
@@ -868,8 +862,7 @@ extern "C" int dsv4_indexer_topk_fwd(const Dsv4IndexerTopkParams* p, void* strea
     e = ensure_smem(indexer_logits_kernel, kIdxSmemBytes, done);
     if (e != cudaSuccess) return int(e);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    indexer_logits_kernel<<<dim3(grid_x, p->B), kIdxThreads, kIdxSmemBytes, s>>>(a);
-    e = cudaGetLastError();
+    e = launch(indexer_logits_kernel, dim3(grid_x, p->B), kIdxThreads, kIdxSmemBytes, s, a);
     if (e != cudaSuccess) return int(e);
     TopkArgs t{};
     t.rows = p->B * p->s_q;  t.k = p->k;  t.scores = p->scores;  t.stride = p->score_stride;  t.n_vis = p->n_vis;
@@ -882,21 +875,6 @@ extern "C" int dsv4_indexer_topk_fwd(const Dsv4IndexerTopkParams* p, void* strea
     static std::atomic<bool> done_topk[kMaxDevices], done_pair[kMaxDevices];
     e = pair ? ensure_smem(topk_select_pair_kernel, 180 * 1024, done_pair) : ensure_smem(topk_select_kernel, 180 * 1024, done_topk);
     if (e != cudaSuccess) return int(e);
-    if (g_dbg.load(std::memory_order_relaxed) & 64) {
-        if (pair) topk_select_pair_kernel<<<t.rows * 2, kTopkThreads, t.row_in_smem ? row_bytes : 0, s>>>(t);
-        else topk_select_kernel<<<t.rows, kTopkThreads, t.row_in_smem ? row_bytes : 0, s>>>(t);
-        return int(cudaGetLastError());
-    }
-    // as a programmatic dependent of the scoring kernel: resident (and waiting) when its last blocks finish
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(pair ? t.rows * 2 : t.rows);
-    cfg.blockDim = dim3(kTopkThreads);
-    cfg.dynamicSmemBytes = t.row_in_smem ? row_bytes : 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return int(pair ? cudaLaunchKernelEx(&cfg, topk_select_pair_kernel, t) : cudaLaunchKernelEx(&cfg, topk_select_kernel, t));
+    return int(launch(pair ? topk_select_pair_kernel : topk_select_kernel, dim3(pair ? t.rows * 2 : t.rows), kTopkThreads,
+                      t.row_in_smem ? row_bytes : 0, s, t));
 }

@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
     __shared__ float sm_l[kHcaRowGroups - 1][kHcaVecsPerBlock][8];
     __shared__ float sm_acc[kHcaRowGroups - 1][kHcaVecsPerBlock][8];
     constexpr float kLog2e = 1.4426950408889634f;
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     const int t = threadIdx.x;
     const int vl = t % kHcaVecsPerBlock, rg = t / kHcaVecsPerBlock;
     const int v = blockIdx.y * kHcaVecsPerBlock + vl;
@@ -254,6 +256,8 @@ constexpr int kInsertThreads = 256;
 // One warp per row: lane l owns latent elements [16 l, 16 l + 16) and RoPE
 // elements [2 l, 2 l + 2); 8 lanes make one 128-element scale block.
 __global__ void __launch_bounds__(kInsertThreads) kv_quantize_insert_kernel(const KvInsertArgs a) {
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t total = int64_t(a.B) * a.T;
     for (int64_t row = int64_t(blockIdx.x) * (kInsertThreads / 32) + (threadIdx.x >> 5); row < total;

@@ -62,6 +62,8 @@ template <> struct BfVec<4> {
 // VEC = 8 / 4: 16- / 8-byte vectors (c_out % VEC == 0 and rows aligned to the vector); VEC = 1: any c_out.
 template <int M, int VEC>
 __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 4 : 2) compress_reduce_kernel(const CompressReduceArgs a) {
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     const int vecs = a.c_out / VEC;
     const int64_t total = int64_t(a.B) * a.n_blocks * vecs;
     for (int64_t idx = int64_t(blockIdx.x) * kCompressThreads + threadIdx.x; idx < total;

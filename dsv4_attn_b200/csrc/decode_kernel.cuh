@@ -656,13 +656,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     const int rows = a.B * a.s_q;
     const uint32_t wait_ns = a.wait_ns;
 
-    // ── this pair's items ──
+    // ── this pair's items (known after set-up) ──
     int item_begin = 0, n_items = 1;
-    if (sched) {
-        const int pair = blockIdx.x >> 1;
-        item_begin = __ldg(a.sched_pair_begin + pair);
-        n_items = __ldg(a.sched_pair_begin + pair + 1) - item_begin;
-    }
     auto get_item = [&](int k) -> Item {
         Item it;
         if (sched) {
@@ -731,6 +726,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     // The barriers of both blocks are initialised before any role of either starts.
     __syncwarp();
     ptx::cluster_sync();
+    ptx::pdl_wait();
+    if (sched) {
+        const int pair = blockIdx.x >> 1;
+        item_begin = __ldg(a.sched_pair_begin + pair);
+        n_items = __ldg(a.sched_pair_begin + pair + 1) - item_begin;
+    }
     // All 512 columns are allocated, so tensor memory starts at address 0 (checked where it is allocated): as a constant it keeps the
     // operands of every tcgen05 instruction out of vector registers.
     constexpr uint32_t tmem = 0;
@@ -1263,9 +1264,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             l_sum += misc->exch[tid ^ 64];
             ptx::tc_fence_after_sync();
             if (tid == 0) trace_mark(a, 0, 4 * int(gt - 1u) + 3);
-            // A merge kernel launched as a programmatic dependent may be made resident once every block of
-            // this grid is here (or gone): by then no block of this grid is waiting for an SM any more.
-            if (tid == 0 && k == n_items - 1 && (sched || a.num_splits > 1)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            // The next kernel (the merge, or the next layer's) may be made resident once every block of this grid is here (or gone): by
+            // then no block of this grid is waiting for an SM any more.
+            if (tid == 0 && k == n_items - 1) ptx::pdl_trigger();
             float denom = l_sum;
             if (final_out && a.attn_sink != nullptr && write) {
                 const float s2 = __ldg(a.attn_sink + h0 + r) * 1.4426950408889634f;

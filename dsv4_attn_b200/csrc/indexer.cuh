@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
     const int b = blockIdx.y;
     const int N = a.s_q * kIdxHeads;
 
+    ptx::pdl_wait();
     int vis_max = 0;
     for (int t = 0; t < a.s_q; ++t) vis_max = max(vis_max, __ldg(a.n_vis + b * a.s_q + t));
     vis_max = min(vis_max, a.max_pages * kIdxPageKeys);
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
     ptx::tc_fence_before_sync();
     __syncthreads();
     // the top-k kernel may be made resident as soon as every block of this grid is here or gone
-    if (tid == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid == 0) ptx::pdl_trigger();
     if (warp == 1) {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem, kIdxTmemCols);
@@ -506,13 +507,15 @@ __device__ __forceinline__ void topk_select_body(const TopkArgs& a, float* topk_
 
 __global__ void __launch_bounds__(kTopkThreads) topk_select_kernel(const TopkArgs a) {
     extern __shared__ float topk_row[];
-    asm volatile("griddepcontrol.wait;" ::: "memory");     // launched as a programmatic dependent of the scoring kernel
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     topk_select_body<1>(a, topk_row);
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTopkThreads) topk_select_pair_kernel(const TopkArgs a) {
     extern __shared__ float topk_row[];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     topk_select_body<2>(a, topk_row);
 }
 

@@ -27,6 +27,14 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
     return t;
 }
 
+// ── programmatic dependent launch ───────────────────────────────────────
+// The library's kernels are launched so that a kernel may start while the one before it in the stream is still draining:
+// its launch and set-up are hidden.  Every kernel therefore waits before it touches memory (returns at once where there
+// is nothing to wait for; after it all earlier work of the stream is complete and visible), and says early that its own
+// successor may be made resident once all of its blocks run.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ── mbarrier ────────────────────────────────────────────────────────────
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

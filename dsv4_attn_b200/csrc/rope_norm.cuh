@@ -36,6 +36,8 @@ constexpr int kRopeNormThreads = 256;
 constexpr int kRopeGroup = 4;           // vectors of one row handled by one warp
 
 __global__ void __launch_bounds__(kRopeNormThreads) rope_norm_kernel(const RopeNormArgs a) {
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     const int lane = threadIdx.x & 31;
     const int nope = a.c - a.n_rope;
     const int half = a.n_rope >> 1;        // 32: one rotated pair per lane

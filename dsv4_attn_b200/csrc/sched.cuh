@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanArgs p) {
     __shared__ int s_count[kPlanMaxPairs];
     __shared__ int s_begin[kPlanMaxPairs + 1];
     __shared__ int s_slots, s_over;
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int n_units = p.rows * p.hgs;
     if (tid == 0) { s_carry = 0;  s_max = 0;  s_slots = 0;  s_over = 0; }
