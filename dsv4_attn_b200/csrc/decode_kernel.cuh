@@ -1264,9 +1264,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             l_sum += misc->exch[tid ^ 64];
             ptx::tc_fence_after_sync();
             if (tid == 0) trace_mark(a, 0, 4 * int(gt - 1u) + 3);
-            // The next kernel (the merge, or the next layer's) may be made resident once every block of this grid is here (or gone): by
-            // then no block of this grid is waiting for an SM any more.
-            if (tid == 0 && k == n_items - 1) ptx::pdl_trigger();
+            // The merge may be made resident once every block of this grid is here (or gone): by then no block of this grid is waiting for
+            // an SM any more.  (Without a merge the successor may be another decode; its blocks, let in this early, cost 2 us of 63.)
+            if (tid == 0 && k == n_items - 1 && (sched || a.num_splits > 1)) ptx::pdl_trigger();
             float denom = l_sum;
             if (final_out && a.attn_sink != nullptr && write) {
                 const float s2 = __ldg(a.attn_sink + h0 + r) * 1.4426950408889634f;
