@@ -8,6 +8,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cmath>
+#include <cstring>
 #include <atomic>
 
 #include "combine.cuh"
@@ -246,6 +247,11 @@ cudaError_t launch_simt(const DecodeArgs& a, int rows, int max_tok, cudaStream_t
 }
 
 cudaError_t launch_combine(const CombineArgs& c, cudaStream_t stream) {
+    if (c.unit_nsplits != nullptr) {      // resident blocks (four per SM) share out what the plan cut, but no more than could have work
+        const int64_t most = int64_t(c.N) * c.hgs * ((c.H < 128 ? c.H : 128) + kCombineWarps - 1) / kCombineWarps;
+        const int64_t resident = int64_t(device_sms()) * 4;
+        return launch(combine_sched_kernel, dim3(unsigned(most < resident ? most : resident)), kCombineWarps * 32, 0, stream, c);
+    }
     const int64_t units = int64_t(c.N) * c.H;
     return launch(combine_kernel, dim3(unsigned((units + kCombineWarps - 1) / kCombineWarps)), kCombineWarps * 32, 0, stream, c);
 }
@@ -798,11 +804,24 @@ extern "C" int dsv4_rope_norm_fwd(const Dsv4RopeNormParams* p, void* stream) {
     a.out = static_cast<__nv_bfloat16*>(p->out);
     a.positions = p->positions;
     a.weight = static_cast<const __nv_bfloat16*>(p->norm_weight);
-    const int sms = device_sms();
-    const int64_t items = a.n_rows * ((a.vecs_per_row + kRopeGroup - 1) / kRopeGroup);
+    // frequency of pair i, 1 / theta^(2 i / n_rope), in double before the rounding to FP32; kept per thread for the theta last used
+    static thread_local float known_theta = 0.f, known_freq[32];
+    if (known_theta != a.theta) {
+        for (int i = 0; i < 32; ++i) known_freq[i] = float(1.0 / std::pow(double(a.theta), double(2 * i) / 64.0));
+        known_theta = a.theta;
+    }
+    std::memcpy(a.freq, known_freq, sizeof(known_freq));
+    // Vectors of a row per warp: as many as still leave every SM eight warps, the number that hides a load's latency
+    // (a larger group computes the angles once for more vectors and keeps more loads in flight per warp).
+    const int64_t fill = int64_t(device_sms()) * 8;
+    int group = 1;
+    if (a.vecs_per_row >= 4 && a.n_rows * ((a.vecs_per_row + 3) / 4) >= fill) group = 4;
+    else if (a.vecs_per_row >= 2 && a.n_rows * ((a.vecs_per_row + 1) / 2) >= fill) group = 2;
+    const int64_t items = a.n_rows * ((a.vecs_per_row + group - 1) / group);
     const int64_t want = (items + kRopeNormThreads / 32 - 1) / (kRopeNormThreads / 32);
-    const int64_t cap = int64_t(sms) * 8;
-    return int(launch(rope_norm_kernel, dim3(unsigned(want < cap ? want : cap)), kRopeNormThreads, 0, static_cast<cudaStream_t>(stream), a));
+    const int64_t cap = fill;
+    auto kernel = group == 4 ? rope_norm_kernel<4> : (group == 2 ? rope_norm_kernel<2> : rope_norm_kernel<1>);
+    return int(launch(kernel, dim3(unsigned(want < cap ? want : cap)), kRopeNormThreads, 0, static_cast<cudaStream_t>(stream), a));
 }
 
 

@@ -48,32 +48,9 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-__global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const CombineArgs a) {
-    ptx::pdl_trigger();
-    ptx::pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t unit = int64_t(blockIdx.x) * kCombineWarps + warp;   // (row, head) flattened
-    if (unit >= int64_t(a.N) * a.H) return;
-    const int n = int(unit / a.H), h = int(unit % a.H);
-    int S = a.num_splits;
-    const float* pl;
-    int64_t pl_stride, po_off, po_stride;      // po_*: element offsets into partial_o (FP32 or BF16 elements)
-    if (a.unit_nsplits != nullptr) {
-        const int u = n * a.hgs + (h >> 7);
-        S = __ldg(a.unit_nsplits + u);
-        if (S <= 1) return;
-        const int64_t row = int64_t(__ldg(a.unit_slot + u)) * 128 + (h & 127);
-        pl = a.partial_lse + row;
-        pl_stride = 128;
-        po_off = row * 512 + lane * 8;
-        po_stride = 128 * 512;
-    } else {
-        pl = a.partial_lse + int64_t(n) * a.stride_pl_n + h;
-        pl_stride = a.stride_pl_split;
-        po_off = int64_t(n) * a.stride_po_n + int64_t(h) * a.stride_po_h + lane * 8;
-        po_stride = a.stride_po_split;
-    }
-
+// One (row, head): its S partial rows of 512 columns, po_stride elements apart from po_off, under the LSEs at pl.
+__device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, int lane, int S, const float* pl, int64_t pl_stride,
+                                           int64_t po_off, int64_t po_stride) {
     // pass 1: maximum and sum over splits.  The first 32 LSEs are loaded once (one per lane) and serve the maximum,
     // the sum and the weights; only rows with more than 32 splits go back to memory.
     const float l_first = (lane < S) ? __ldg(pl + int64_t(lane) * pl_stride) : -CUDART_INF_F;
@@ -175,6 +152,70 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const Combi
         w.z = ptx::pack_bf16x2(acc[i][4], acc[i][5]);
         w.w = ptx::pack_bf16x2(acc[i][6], acc[i][7]);
         *reinterpret_cast<uint4*>(dst + i * 256) = w;
+    }
+}
+
+// Every (row, head) has num_splits partials.
+__global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __grid_constant__ CombineArgs a) {
+    ptx::pdl_trigger();
+    ptx::pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t unit = int64_t(blockIdx.x) * kCombineWarps + warp;   // (row, head) flattened
+    if (unit >= int64_t(a.N) * a.H) return;
+    const int n = int(unit / a.H), h = int(unit % a.H);
+    merge_head(a, n, h, lane, a.num_splits, a.partial_lse + int64_t(n) * a.stride_pl_n + h, a.stride_pl_split,
+               int64_t(n) * a.stride_po_n + int64_t(h) * a.stride_po_h + lane * 8, a.stride_po_split);
+}
+
+// After a scheduled decode.  A plan cuts at most as many units as there are block pairs, usually far fewer than the batch has, so
+// the grid is what is resident at once and its blocks share the cut units out, eight heads at a time: each block gathers them from
+// the plan's list (256 requests, mixed lengths: 12.5 -> 10 us cold against one warp per (row, head) of the batch, of which nine in ten had nothing to do).
+__global__ void __launch_bounds__(kCombineWarps * 32) combine_sched_kernel(const __grid_constant__ CombineArgs a) {
+    constexpr int kPerThread = 4, kChunk = kCombineWarps * 32 * kPerThread;
+    __shared__ int s_unit[kChunk];
+    __shared__ int s_count[kCombineWarps];
+    ptx::pdl_trigger();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n_units = a.N * a.hgs;
+    const int slices = (min(a.H, 128) + kCombineWarps - 1) / kCombineWarps;
+    int64_t job0 = 0;                         // jobs (cut unit, eight heads) of the chunks before this one
+    for (int base = 0; base < n_units; base += kChunk) {
+        // The plan is read ahead of the wait below: the decode kernel, whose blocks have all started by now, waited for it.
+        uint32_t cut[kPerThread];             // which units of the warp's 128 are cut
+        int mine = 0;
+#pragma unroll
+        for (int i = 0; i < kPerThread; ++i) {
+            const int u = base + (warp * kPerThread + i) * 32 + lane;
+            cut[i] = __ballot_sync(0xFFFFFFFFu, u < n_units && __ldg(a.unit_nsplits + u) > 1);
+            mine += __popc(cut[i]);
+        }
+        __syncthreads();                      // the chunk before is done with the list
+        if (lane == 0) s_count[warp] = mine;
+        __syncthreads();
+        int at = 0, count = 0;
+#pragma unroll
+        for (int w = 0; w < kCombineWarps; ++w) {
+            if (w < warp) at += s_count[w];
+            count += s_count[w];
+        }
+#pragma unroll
+        for (int i = 0; i < kPerThread; ++i) {
+            if (cut[i] >> lane & 1u) s_unit[at + __popc(cut[i] & ((1u << lane) - 1u))] = base + (warp * kPerThread + i) * 32 + lane;
+            at += __popc(cut[i]);
+        }
+        __syncthreads();
+        const int jobs = count * slices;
+        if (base == 0) ptx::pdl_wait();
+        int64_t first = (int64_t(blockIdx.x) - job0) % int64_t(gridDim.x);
+        if (first < 0) first += gridDim.x;
+        for (int64_t j = first; j < jobs; j += gridDim.x) {
+            const int u = s_unit[j / slices], n = u / a.hgs;
+            const int in_group = int(j % slices) * kCombineWarps + warp, h = (u % a.hgs) * 128 + in_group;
+            if (h >= a.H) continue;
+            const int64_t row = int64_t(__ldg(a.unit_slot + u)) * 128 + in_group;
+            merge_head(a, n, h, lane, __ldg(a.unit_nsplits + u), a.partial_lse + row, 128, row * 512 + lane * 8, 128 * 512);
+        }
+        job0 += jobs;
     }
 }
 

@@ -79,6 +79,12 @@ __host__ __device__ __forceinline__ bool plan_keep_whole(int n_units, int num_pa
     return t_whole <= quota + kPlanMergeCost;
 }
 
+// x / d for what fits 32 bits (nearly always), in a 32-bit division: a 64-bit one is a subroutine of some 100 instructions.
+__host__ __device__ __forceinline__ long long plan_div(long long x, long long d) {
+    if (((unsigned long long)(x | d) >> 32) == 0) return (long long)((unsigned)x / (unsigned)d);
+    return x / d;
+}
+
 // Walks the pieces of the unit that starts at C on the cost axis: next() yields (pair, first tile, tiles)
 // of one piece after the other.
 struct PieceWalk {
@@ -86,7 +92,7 @@ struct PieceWalk {
     int cost, tiles, last_pair, fixed, tps, t, pr, p1;
     bool single, done;
     __host__ __device__ int pair_of(long long x) const {
-        const long long q = x / quota;
+        const long long q = plan_div(x, quota);
         return int(q < last_pair ? q : last_pair);
     }
     __host__ __device__ PieceWalk(const PlanArgs& p, long long C_, int cost_, int tiles_, long long quota_, bool whole)
@@ -121,7 +127,7 @@ struct PieceWalk {
         while (pr <= p1) {
             const long long lo = (pr == p0) ? 0 : (long long)pr * quota - C;
             const long long hi = (pr == p1) ? cost : (long long)(pr + 1) * quota - C;
-            const int ta = int((lo * tiles + cost / 2) / cost), tb = int((hi * tiles + cost / 2) / cost);
+            const int ta = int(plan_div(lo * tiles + cost / 2, cost)), tb = int(plan_div(hi * tiles + cost / 2, cost));
             const int here = pr++;
             if (tb > ta) {
                 pair = here;  t0 = ta;  nt = tb - ta;
@@ -133,69 +139,81 @@ struct PieceWalk {
     }
 };
 
-__global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanArgs p) {
+// Inclusive sum of v over the block; warp_sums is scratch of 32.
+template <class T>
+__device__ __forceinline__ T plan_block_scan(T v, T* warp_sums) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += t;
+    }
+    if (lane == 31) warp_sums[wid] = v;
+    __syncthreads();
+    T before = lane < wid ? warp_sums[lane] : T(0);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
+    return v + before;
+}
+
+// One block: the time is the chain of its steps (load, scan, deal, scan, write), not bandwidth.  A thread keeps the lengths, cost and
+// prefix of its first unit in registers from pass to pass (all there are up to 1024 units), both sums are block scans, and
+// the divisions are 32-bit where they can be: 256 rows take xx us (9.3 with one thread adding up the pairs and everything read back from memory).
+__global__ void __launch_bounds__(kPlanThreads) plan_kernel(const __grid_constant__ PlanArgs p) {
     __shared__ long long s_warp[32];
+    __shared__ int s_warp_i[32];
     __shared__ long long s_carry;
     __shared__ int s_max;
     __shared__ int s_count[kPlanMaxPairs];
     __shared__ int s_begin[kPlanMaxPairs + 1];
     __shared__ int s_slots, s_over;
     ptx::pdl_trigger();
-    ptx::pdl_wait();
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int n_units = p.rows * p.hgs;
     if (tid == 0) { s_carry = 0;  s_max = 0;  s_slots = 0;  s_over = 0; }
-    for (int i = tid; i < p.num_pairs; i += kPlanThreads) s_count[i] = 0;
+    s_count[tid] = 0;
+    ptx::pdl_wait();
     __syncthreads();
+
+    struct Unit { int row, n_tok, kv_len_n, tiles, cost; };
+    auto read_unit = [&](int u) {
+        Unit x;
+        x.row = u / p.hgs;
+        plan_row_lengths(p, x.row, x.n_tok, x.kv_len_n);
+        x.tiles = (x.n_tok + kTileN - 1) / kTileN;
+        x.cost = plan_unit_cost(x.tiles, p.fixed_splits);
+        return x;
+    };
+    Unit first{};
+    long long first_prefix = 0;
+    int first_slot = -1;
 
     // pass 1: cost of every unit and its start on the cost axis
     for (int base = 0; base < n_units; base += kPlanThreads) {
         const int u = base + tid;
-        int cost = 0;
-        if (u < n_units) {
-            int n_tok, kv_len_n;
-            plan_row_lengths(p, u / p.hgs, n_tok, kv_len_n);
-            cost = plan_unit_cost((n_tok + kTileN - 1) / kTileN, p.fixed_splits);
-            atomicMax(&s_max, cost);
-        }
-        long long incl = cost;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) s_warp[wid] = incl;
+        Unit x{};
+        if (u < n_units) x = read_unit(u);
+        const int warp_max = __reduce_max_sync(0xFFFFFFFFu, x.cost);
+        if (lane == 0) atomicMax(&s_max, warp_max);
+        const long long before = s_carry + plan_block_scan<long long>(x.cost, s_warp) - x.cost;
+        if (base == 0) { first = x;  first_prefix = before; }
+        else if (u < n_units) p.unit_prefix[u] = before;
         __syncthreads();
-        if (wid == 0) {
-            long long w = s_warp[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long t = __shfl_up_sync(0xFFFFFFFFu, w, o);
-                if (lane >= o) w += t;
-            }
-            s_warp[lane] = w;
-        }
-        __syncthreads();
-        const long long before = s_carry + (wid > 0 ? s_warp[wid - 1] : 0) + incl - cost;
-        if (u < n_units) p.unit_prefix[u] = before;
-        __syncthreads();
-        if (tid == kPlanThreads - 1) s_carry = before + cost;
+        if (tid == kPlanThreads - 1) s_carry = before + x.cost;
         __syncthreads();
     }
     const long long total = s_carry;
-    long long quota = (total + p.num_pairs - 1) / p.num_pairs;
+    long long quota = plan_div(total + p.num_pairs - 1, p.num_pairs);
     if (quota < 1) quota = 1;
     const bool whole = plan_keep_whole(n_units, p.num_pairs, s_max, quota);
 
     // pass 2: pieces per pair, pieces per unit, partial slots
     for (int u = tid; u < n_units; u += kPlanThreads) {
-        int n_tok, kv_len_n;
-        plan_row_lengths(p, u / p.hgs, n_tok, kv_len_n);
-        const int tiles = (n_tok + kTileN - 1) / kTileN;
-        const int cost = plan_unit_cost(tiles, p.fixed_splits);
+        const bool kept = u == tid;
+        const Unit x = kept ? first : read_unit(u);
         int pieces = 0;
         {
-            PieceWalk w(p, p.unit_prefix[u], cost, tiles, quota, whole);
+            PieceWalk w(p, kept ? first_prefix : p.unit_prefix[u], x.cost, x.tiles, quota, whole);
             int pr, t0, nt;
             while (w.next(pr, t0, nt)) { atomicAdd(&s_count[pr], 1);  ++pieces; }
         }
@@ -204,24 +222,31 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanArgs p) {
             slot = atomicAdd(&s_slots, pieces);
             if (slot + pieces > p.slot_cap) { s_over = 1;  slot = -1; }
         }
+        if (kept) first_slot = slot;
         p.unit_nsplits[u] = pieces;
         p.unit_slot[u] = slot;
     }
     __syncthreads();
 
     // pass 3: first item of every pair
-    if (tid == 0) {
-        int acc = 0;
-        for (int i = 0; i < p.num_pairs; ++i) { s_begin[i] = acc;  acc += s_count[i];  s_count[i] = 0; }
-        s_begin[p.num_pairs] = acc;
-        if (acc > p.item_cap) s_over = 1;
+    {
+        const int mine = s_count[tid];                       // zero from num_pairs on
+        const int upto = plan_block_scan<int>(mine, s_warp_i);
+        s_begin[tid] = upto - mine;
+        s_count[tid] = 0;
+        if (tid == kPlanThreads - 1) {
+            s_begin[kPlanMaxPairs] = upto;
+            if (upto > p.item_cap) s_over = 1;
+        }
     }
     __syncthreads();
     const bool over = s_over != 0;
+    const int n_items = s_begin[kPlanMaxPairs];
     // (pairs beyond num_pairs - a launch with more blocks than the plan was made for - find empty lists)
-    for (int i = tid; i <= kPlanMaxPairs; i += kPlanThreads) p.pair_begin[i] = over ? 0 : s_begin[i < p.num_pairs ? i : p.num_pairs];
+    p.pair_begin[tid] = over ? 0 : s_begin[tid];
     if (tid == 0) {
-        p.info[0] = s_begin[p.num_pairs];
+        p.pair_begin[kPlanMaxPairs] = over ? 0 : n_items;
+        p.info[0] = n_items;
         p.info[1] = s_slots;
         p.info[2] = over ? 1 : 0;
         p.info[3] = int(quota < 0x7FFFFFFF ? quota : 0x7FFFFFFF);
@@ -230,23 +255,21 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanArgs p) {
 
     // pass 4: the items
     for (int u = tid; u < n_units; u += kPlanThreads) {
-        const int row = u / p.hgs, hg = u % p.hgs;
-        int n_tok, kv_len_n;
-        plan_row_lengths(p, row, n_tok, kv_len_n);
-        const int tiles = (n_tok + kTileN - 1) / kTileN;
-        const int cost = plan_unit_cost(tiles, p.fixed_splits);
-        const int slot0 = p.unit_slot[u];
-        PieceWalk w(p, p.unit_prefix[u], cost, tiles, quota, whole);
+        const bool kept = u == tid;
+        const Unit x = kept ? first : read_unit(u);
+        const int slot0 = kept ? first_slot : p.unit_slot[u];
+        PieceWalk w(p, kept ? first_prefix : p.unit_prefix[u], x.cost, x.tiles, quota, whole);
         int pr, t0, nt, j = 0;
         while (w.next(pr, t0, nt)) {
             const int at = s_begin[pr] + atomicAdd(&s_count[pr], 1);
             int4* rec = reinterpret_cast<int4*>(p.items + int64_t(at) * kItemWords);
-            rec[0] = make_int4(row, hg, t0, nt);
-            rec[1] = make_int4(slot0 >= 0 ? slot0 + j : -1, n_tok, kv_len_n, 0);
+            rec[0] = make_int4(x.row, u % p.hgs, t0, nt);
+            rec[1] = make_int4(slot0 >= 0 ? slot0 + j : -1, x.n_tok, x.kv_len_n, 0);
             ++j;
         }
     }
 }
+static_assert(kPlanThreads == kPlanMaxPairs, "one thread per pair");
 
 // The same plan computed serially on the host from length arrays in host memory (every pointer of `p`
 // is then a host pointer).  For inspection and for tests of the planning arithmetic without a GPU; the
@@ -263,7 +286,7 @@ inline void plan_host(const PlanArgs& p) {
         total += cost;
         if (cost > max_cost) max_cost = cost;
     }
-    long long quota = (total + p.num_pairs - 1) / p.num_pairs;
+    long long quota = plan_div(total + p.num_pairs - 1, p.num_pairs);
     if (quota < 1) quota = 1;
     const bool whole = plan_keep_whole(n_units, p.num_pairs, max_cost, quota);
     for (int i = 0; i <= kPlanMaxPairs; ++i) p.pair_begin[i] = 0;
