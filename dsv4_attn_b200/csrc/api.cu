@@ -679,8 +679,8 @@ extern "C" int dsv4_csa_compress_reduce_fwd(const Dsv4CsaCompressReduceParams* p
     const int sms = device_sms();
     const int64_t items = int64_t(a.B) * a.n_blocks * (vec ? a.c_out / 4 : a.c_out);
     const int64_t want = (items + kCompressThreads - 1) / kCompressThreads;
-    // at most 8 blocks per SM (two waves of the 4 resident ones); beyond that the grid-stride loop takes over
-    const int64_t cap = int64_t(sms) * 8;
+    // at most 6 blocks per SM (two waves of the 3 resident ones); beyond that the grid-stride loop takes over
+    const int64_t cap = int64_t(sms) * 6;
     const int blocks = int(want < cap ? (want > 0 ? want : 1) : cap);
     return int(launch(vec ? compress_reduce_kernel<4, 4> : compress_reduce_kernel<4, 1>, dim3(blocks), kCompressThreads, 0,
                       static_cast<cudaStream_t>(stream), a));

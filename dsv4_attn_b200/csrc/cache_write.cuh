@@ -60,7 +60,8 @@ __device__ __forceinline__ float block_scale(float absmax) {
 }
 
 // x / scale from the correctly rounded reciprocal r = RN(1 / scale): one multiply, the
-// remainder by FMA, one corrective FMA (the classical FMA division step).  Three instructions
+// remainder by FMA, one corrective FMA (Markstein's division step for machines with a fused multiply-add: P. Markstein,
+// IBM Journal of Research and Development 34(1), 1990).  Three instructions
 // instead of the dozen of a general division, whose range handling is not needed here: scale is
 // a normal number and |x / scale| <= 448.  The step reproduced the IEEE quotient on every one of
 // 8e7 random (x, scale) pairs checked on the CPU; a last-bit difference could change the e4m3

@@ -3,10 +3,11 @@
 // previous block on the b-side, each plus a per-position bias) weights the 2m
 // value rows.  A pure streaming kernel: every input element is read once with
 // vector loads, one thread owns 4 consecutive channels of one output block (8-byte loads: a
-// thread then holds 16 vectors = 32 registers of raw data, four blocks fit an SM, and the 32
-// resident warps hide each other's arithmetic phase; with 8 channels per thread and two blocks
-// per SM the kernel was 7 % slower, with 2 channels and five blocks 30 % slower), and the grid
-// is sized so that all SMs hold two waves of resident blocks.
+// thread then holds 16 vectors = 32 registers of raw data).  Bound by HBM and, close behind, by instruction issue: the
+// arithmetic is done two channels at a time (packed BF16 for the reference maximum, packed FP32 for the rest), 230
+// instructions a thread instead of 420, and three blocks fit an SM at 80 registers (at four and 64 registers it
+// spills: 34 us).  32k rows: 34 -> 30 us, 5.0 TB/s.  The grid is sized so that all SMs hold two waves
+// of resident blocks.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -61,7 +62,7 @@ template <> struct BfVec<4> {
 
 // VEC = 8 / 4: 16- / 8-byte vectors (c_out % VEC == 0 and rows aligned to the vector); VEC = 1: any c_out.
 template <int M, int VEC>
-__global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 4 : 2) compress_reduce_kernel(const CompressReduceArgs a) {
+__global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_reduce_kernel(const CompressReduceArgs a) {
     ptx::pdl_trigger();
     ptx::pdl_wait();
     const int vecs = a.c_out / VEC;
@@ -94,48 +95,63 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 4 : 2) compress_r
                     cb[j] = BfVec<VEC>::load_stream(a.C_b + row_b + j * a.stride_c_n);
                 }
             }
-            auto logits = [&](int j, bool bside, float (&z)[VEC]) {
-                float u[VEC];
-                BfVec<VEC>::unpack(bside ? zb[j] : za[j], z);
-                BfVec<VEC>::unpack(__ldg(reinterpret_cast<const V*>((bside ? a.B_b : a.B_a) + int64_t(j) * a.c_out + ch)), u);
+            auto bias = [&](int j, bool bside) { return __ldg(reinterpret_cast<const V*>((bside ? a.B_b : a.B_a) + int64_t(j) * a.c_out + ch)); };
+            // The reference maximum is found in packed BF16 arithmetic: any value close to the true maximum serves, as long as the
+            // same one is used for every weight.  The logits themselves are formed in FP32, two channels an instruction.
+            constexpr int P = VEC / 2;
+            __nv_bfloat162 pm[P];
 #pragma unroll
-                for (int k = 0; k < VEC; ++k) z[k] += u[k];
-            };
-            float zmax[VEC], sum[VEC], acc[VEC];
-#pragma unroll
-            for (int k = 0; k < VEC; ++k) { zmax[k] = -CUDART_INF_F;  sum[k] = 0.f;  acc[k] = 0.f; }
+            for (int k = 0; k < P; ++k) pm[k] = __float2bfloat162_rn(-CUDART_INF_F);
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
                 if (side == 1 && !has_b) break;
 #pragma unroll
                 for (int j = 0; j < M; ++j) {
-                    float z[VEC];
-                    logits(j, side == 1, z);
+                    const V z = side ? zb[j] : za[j], u = bias(j, side == 1);
+                    const __nv_bfloat162 *z2 = reinterpret_cast<const __nv_bfloat162*>(&z), *u2 = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
-                    for (int k = 0; k < VEC; ++k) zmax[k] = fmaxf(zmax[k], z[k]);
+                    for (int k = 0; k < P; ++k) pm[k] = __hmax2(pm[k], __hadd2(z2[k], u2[k]));
                 }
             }
+            constexpr float kLog2e = 1.4426950408889634f;
+            const uint64_t log2e2 = ptx::pack_f32x2(kLog2e, kLog2e);
+            uint64_t nref[P], sum2[P], acc2[P];             // nref: -(reference maximum) * log2(e)
 #pragma unroll
-            for (int k = 0; k < VEC; ++k)
-                if (!(zmax[k] > -CUDART_INF_F) || !(zmax[k] < CUDART_INF_F)) zmax[k] = 0.f;   // all -inf (or NaN): avoid inf - inf
+            for (int k = 0; k < P; ++k) {
+                float lo = __low2float(pm[k]), hi = __high2float(pm[k]);
+                if (!(lo > -CUDART_INF_F) || !(lo < CUDART_INF_F)) lo = 0.f;   // all -inf (or NaN): avoid inf - inf
+                if (!(hi > -CUDART_INF_F) || !(hi < CUDART_INF_F)) hi = 0.f;
+                nref[k] = ptx::pack_f32x2(-lo * kLog2e, -hi * kLog2e);
+                sum2[k] = 0ull;  acc2[k] = 0ull;
+            }
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
                 if (side == 1 && !has_b) break;
 #pragma unroll
                 for (int j = 0; j < M; ++j) {
-                    float z[VEC], c[VEC];
-                    logits(j, side == 1, z);
-                    BfVec<VEC>::unpack(side == 1 ? cb[j] : ca[j], c);
+                    float z[VEC], u[VEC], c[VEC];
+                    BfVec<VEC>::unpack(side ? zb[j] : za[j], z);
+                    BfVec<VEC>::unpack(bias(j, side == 1), u);
+                    BfVec<VEC>::unpack(side ? cb[j] : ca[j], c);
 #pragma unroll
-                    for (int k = 0; k < VEC; ++k) {
-                        const float e = ptx::ex2((z[k] - zmax[k]) * 1.4426950408889634f);
-                        sum[k] += e;
-                        acc[k] = fmaf(e, c[k], acc[k]);
+                    for (int k = 0; k < P; ++k) {
+                        const uint64_t t = ptx::add_f32x2(ptx::pack_f32x2(z[2 * k], z[2 * k + 1]), ptx::pack_f32x2(u[2 * k], u[2 * k + 1]));
+                        float e0, e1;
+                        ptx::unpack_f32x2(ptx::fma_f32x2(t, log2e2, nref[k]), e0, e1);
+                        const uint64_t e = ptx::pack_f32x2(ptx::ex2(e0), ptx::ex2(e1));
+                        sum2[k] = ptx::add_f32x2(sum2[k], e);
+                        acc2[k] = ptx::fma_f32x2(e, ptx::pack_f32x2(c[2 * k], c[2 * k + 1]), acc2[k]);
                     }
                 }
             }
 #pragma unroll
-            for (int k = 0; k < VEC; ++k) o[k] = acc[k] / sum[k];
+            for (int k = 0; k < P; ++k) {
+                float s0, s1, a0, a1;
+                ptx::unpack_f32x2(sum2[k], s0, s1);
+                ptx::unpack_f32x2(acc2[k], a0, a1);
+                o[2 * k] = a0 / s0;
+                o[2 * k + 1] = a1 / s1;
+            }
         } else {
             float z[2 * M], c[2 * M];
 #pragma unroll
