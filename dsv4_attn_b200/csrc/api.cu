@@ -80,31 +80,46 @@ cudaError_t make_row_map(CUtensorMap* map, const void* base, int64_t rows, int p
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// Pages of `tokens` rows of 576 bytes (and 8 bytes of scales per row behind them), by (byte / 4, token, page): box of `box_bytes` of four tokens.
+cudaError_t make_page_map(CUtensorMap* map, const void* base, int64_t pages, int tokens, int box_bytes) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return cudaErrorNotSupported;
+    const cuuint64_t dims[3] = {144, cuuint64_t(tokens), cuuint64_t(pages)};
+    const cuuint64_t strides[2] = {576, cuuint64_t(tokens) * 584};
+    const cuuint32_t box[3] = {cuuint32_t(box_bytes / 4), 4, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 // The record maps of one pool (DecodeArgs::rec_map, rope_map).  A map is a function of the pool's address, rows and kind alone, and a
 // program's pools stay where they are from call to call, so each thread keeps the last few it made (2 us a call otherwise).
 struct PoolMaps {
     const void* lat = nullptr;
     const void* rope = nullptr;
     int64_t rows = 0;
-    bool ref = false;
+    int src = -1, page = 0;
     CUtensorMap rec[3], rope_map;
 };
-cudaError_t pool_maps(const PoolMaps** out, const void* lat, const void* rope, int64_t rows, bool ref) {
+// (page: tokens per page where the rows are pages)
+cudaError_t pool_maps(const PoolMaps** out, const void* lat, const void* rope, int64_t rows, int src, int page) {
     constexpr int kKept = 8;
     static thread_local PoolMaps kept[kKept];
     static thread_local int next = 0;
     for (const PoolMaps& m : kept)
-        if (m.lat == lat && m.rope == rope && m.rows == rows && m.ref == ref) { *out = &m;  return cudaSuccess; }
+        if (m.lat == lat && m.rope == rope && m.rows == rows && m.src == src && m.page == page) { *out = &m;  return cudaSuccess; }
     if (rows > 0x7FFFFFFF) return cudaErrorInvalidValue;                   // TMA coordinates are 32-bit
     PoolMaps& m = kept[next];
     m.lat = nullptr;
-    const int pitch = ref ? 448 : 656;
-    const int boxes[3] = {pitch, 256, ref ? 192 : 16};
+    const bool ref = src == kSrcRef;
+    const int pitch = page ? 576 : (ref ? 448 : 656), boxes[3] = {pitch, 256, page ? 320 : (ref ? 192 : 16)};
     cudaError_t e = cudaSuccess;
-    for (int j = 0; j < 3 && e == cudaSuccess; ++j) e = make_row_map(&m.rec[j], lat, rows, pitch, boxes[j]);
+    for (int j = 0; j < 3 && e == cudaSuccess; ++j)
+        e = page ? make_page_map(&m.rec[j], lat, rows, page, boxes[j]) : make_row_map(&m.rec[j], lat, rows, pitch, boxes[j]);
     if (e == cudaSuccess && ref) e = make_row_map(&m.rope_map, rope, rows, 128, 128);
     if (e != cudaSuccess) return e;
-    m.lat = lat;  m.rope = rope;  m.rows = rows;  m.ref = ref;
+    m.lat = lat;  m.rope = rope;  m.rows = rows;  m.src = src;  m.page = page;
     next = (next + 1) % kKept;
     *out = &m;
     return e;
@@ -113,15 +128,16 @@ cudaError_t pool_maps(const PoolMaps** out, const void* lat, const void* rope, i
 // The record maps of a decode call: pool 0 the cache, pool 1 the window; an absent pool has none.
 template <int SRC>
 cudaError_t make_record_maps(DecodeArgs& a) {
-    if constexpr (SRC == kSrcRefPaged) return cudaSuccess;                 // fetched by untiled copies
-    constexpr bool ref = is_ref_layout(SRC);
+    constexpr bool ref = SRC == kSrcRef, paged = SRC == kSrcRefPaged;
+    // (the CSA and HCA sources read the same records: one set of maps for a pool)
+    constexpr int kind = is_ref_layout(SRC) ? SRC : int(kSrcCsa);
     const struct { const void* lat;  const void* rope;  int64_t rows; } pools[2] = {
-        {ref ? a.ref_kc : a.kv_pool, a.ref_kc_rope, ref ? int64_t(a.B) * a.ref_m_cur : int64_t(a.num_pages) * 64},
-        {ref ? a.ref_ks : a.win_pool, a.ref_ks_rope, ref ? int64_t(a.B) * a.ref_swa_len : int64_t(a.B) * a.win_cap}};
+        {paged ? a.pg_kv : (ref ? a.ref_kc : a.kv_pool), a.ref_kc_rope, paged ? a.pg_num_pages : (ref ? int64_t(a.B) * a.ref_m_cur : int64_t(a.num_pages) * 64)},
+        {paged ? a.pg_swa : (ref ? a.ref_ks : a.win_pool), a.ref_ks_rope, paged ? a.pg_swa_num_pages : (ref ? int64_t(a.B) * a.ref_swa_len : int64_t(a.B) * a.win_cap)}};
     for (int i = 0; i < 2; ++i) {
         if (pools[i].lat == nullptr || pools[i].rows <= 0) continue;
         const PoolMaps* m = nullptr;
-        const cudaError_t e = pool_maps(&m, pools[i].lat, pools[i].rope, pools[i].rows, ref);
+        const cudaError_t e = pool_maps(&m, pools[i].lat, pools[i].rope, pools[i].rows, kind, paged ? 1 << a.pg_page_shift : 0);
         if (e != cudaSuccess) return e;
         for (int j = 0; j < 3; ++j) a.rec_map[i][j] = m->rec[j];
         if (ref) a.rope_map[i] = m->rope_map;

@@ -112,9 +112,11 @@ enum StatusCode : int {
 struct DecodeArgs {
     // TMA descriptor of Q viewed as [rows = B*s_q*H, cols = 64*NCHUNK] bf16, box 64 x 64, 128-byte swizzle
     alignas(64) CUtensorMap q_map;
-    // Record fetch (tile::gather4, 32-bit elements, one row high), per pool (0 cache, 1 window):
+    // Record fetch, per pool (0 cache, 1 window), 32-bit elements.  tile::gather4, one row high:
     //   packed 656-byte records: whole record | 256 bytes of latent | 16 bytes of scales
     //   reference planes: latent row (448) | 256 bytes of it | 192 bytes of it;  RoPE row (128) in rope_map
+    // tiled, four tokens of a page:
+    //   packed reference pages: token (576) | 256 bytes of it | 320 bytes of it
     alignas(64) CUtensorMap rec_map[2][3];
     alignas(64) CUtensorMap rope_map[2];
     int B, s_q, H;
@@ -426,6 +428,35 @@ __device__ __forceinline__ void prefetch_q_l2(const DecodeArgs& a, int n, int hg
     for (int l = lane; l < lines; l += 32) ptx::prefetch_l2(base + int64_t(l) * 128);
 }
 
+// What the chain from a row's lengths to its first records runs through (lengths, index list, block table), and its Q, pulled
+// into L2 at the very start of a launch on the static grid, where the row is known from the grid position: the chain then
+// waits for DRAM once instead of three times.  Nothing is read, so the kernel before may still be writing these.
+template <int NCHUNK, int SRC>
+__device__ __forceinline__ void prefetch_start(const DecodeArgs& a, int n, int hg, int rank, int warp, int lane) {
+    constexpr int kMostLines = 128;
+    auto row = [&](const void* p, int64_t bytes) {
+        const int lines = int(min(bytes, int64_t(kMostLines) * 128));
+#pragma unroll 1
+        for (int at = lane * 128; at < lines; at += 32 * 128) ptx::prefetch_l2(static_cast<const uint8_t*>(p) + at);
+    };
+    const int b = n / a.s_q;
+    if (warp == 0) {
+        if (lane == 0 && a.kv_len != nullptr) ptx::prefetch_l2(a.kv_len + n);
+        if (lane == 1 && a.topk_len != nullptr) ptx::prefetch_l2(a.topk_len + n);
+        if (lane == 2 && a.win_len != nullptr) ptx::prefetch_l2(a.win_len + n);
+    } else if (warp == 1) {
+        if (SRC == kSrcCsa && rank == 0) row(a.indices + int64_t(n) * a.topk, int64_t(a.topk) * 4);
+    } else if (warp == 2) {
+        if (rank == 1) row(a.block_table + int64_t(b) * a.max_pages, int64_t(a.max_pages) * 4);
+    } else {
+        const int h0 = hg * kHeadsPerCta + rank * kHeadsPerBlock;
+        const uint8_t* base = reinterpret_cast<const uint8_t*>(a.q + (int64_t(n) * a.H + h0) * (64 * NCHUNK));
+        const int lines = min(kHeadsPerBlock, a.H - h0) * NCHUNK;
+#pragma unroll 1
+        for (int l = (warp - 3) * 32 + lane; l < lines; l += (kNumVWarps - 3) * 32) ptx::prefetch_l2(base + int64_t(l) * 128);
+    }
+}
+
 // The row lengths of an item, from the per-row length arrays.
 template <int SRC>
 __device__ __forceinline__ void row_lengths(const DecodeArgs& a, int n, int& n_tok, int& kv_len_n) {
@@ -495,12 +526,29 @@ __device__ __forceinline__ void fetch_raw(const DecodeArgs& a, const int32_t* id
                                           uint32_t stage, uint32_t bar, int lane) {
     using R = RawLayout<SRC>;
     if constexpr (SRC == kSrcRefPaged) {
-        // pages are no row-addressable tensor: one bulk copy per token
+        // A group of four rows is one box where its tokens follow one another in one page; at the end of a row, and where a row of
+        // window tokens crosses a page, it is one bulk copy per token.  (32 of those occupy a warp for 2000 cycles.)
         const uint32_t bytes = p == 0 ? 576u : (rank ? 320u : 256u);
-        if (lane == 0) ptx::mbar_arrive_expect_tx(bar, uint32_t(__popc(valid)) * bytes);
+        const int id = ids[lane], id0 = __shfl_sync(0xFFFFFFFFu, id, lane & ~3);
+        const uint32_t swa = (second >> lane) & 1u, swa0 = (second >> (lane & ~3)) & 1u;
+        // (the first test: record numbers follow one another across pages of 64 that do)
+        const uint32_t odd = __ballot_sync(0xFFFFFFFFu, (id0 & 63) > 60 || !((valid >> lane) & 1u) || id != id0 + (lane & 3) || swa != swa0);
+        const uint32_t boxes = ~(odd | (odd >> 1) | (odd >> 2) | (odd >> 3)) & 0x11111111u, single = valid & ~(boxes * 15u);
+        if (lane == 0) ptx::mbar_arrive_expect_tx(bar, uint32_t(4 * __popc(boxes) + __popc(single)) * bytes);
         __syncwarp();
-        if ((valid >> lane) & 1u) {
-            const RecordPtr<SRC> r(a, uint32_t(ids[lane]) | (((second >> lane) & 1u) ? kIdSecond : 0u));
+        if (ptx::elect_one()) {
+            int first[8];
+#pragma unroll
+            for (int g = 0; g < 8; ++g) first[g] = ids[4 * g];
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+                if ((boxes >> (4 * g)) & 1u)
+                    ptx::tma_load_3d(stage + (p == 0 ? R::own(4 * g) : R::half(4 * g, rank)), &a.rec_map[(second >> (4 * g)) & 1u][p == 0 ? 0 : 1 + rank],
+                                     p == 0 ? 0 : 64 * rank, first[g] & 63, first[g] >> 6, bar);
+        }
+        __syncwarp();
+        if ((single >> lane) & 1u) {
+            const RecordPtr<SRC> r(a, uint32_t(id) | (swa ? kIdSecond : 0u));
             ptx::bulk_load(stage + (p == 0 ? R::own(lane) : R::half(lane, rank)), r.lat + (p == 0 ? 0 : 256 * rank), bytes, bar);
         }
         __syncwarp();
@@ -699,7 +747,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         else ptx::mbar_arrive_remote(ptx::mapa(bar, 0));
     };
 
+    // On the static grid a packed-layout launch sees to Q before anything is known of the row.  (The reference planes, with no lengths,
+    // indices or tables to wait for, have their first records before Q: 1 us of 45 slower with Q first.)
+    const bool early_q = use_f16(SRC) && !sched;
+
     // ── set-up ──
+    if (early_q && warp >= kFirstVWarp && warp < kSWarp) prefetch_start<NCHUNK, SRC>(a, blockIdx.y, blockIdx.x >> 1, rank, warp - kFirstVWarp, lane);
+    if (warp == kSWarp && lane == 0) ptx::prefetch_tensormap(&a.q_map);
+    if (!is_ref_layout(SRC) && warp == kFetchWarp && lane < 3 && a.num_pages > 0) ptx::prefetch_tensormap(&a.rec_map[0][lane]);
     if (tid == 0) {
         for (int i = 0; i < kStages; ++i) {
             ptx::mbar_init(bar_raw_full + 8 * i, 2);
@@ -711,7 +766,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         }
         ptx::mbar_init(bar_tmem, 1);
         ptx::mbar_init(bar_v_free, 1);
-        ptx::mbar_init(bar_q_ready, 2 * kNumVWarps);
+        ptx::mbar_init(bar_q_ready, 2 * (early_q ? kNumVWarps + kNumKWarps : kNumVWarps));
         for (int i = 0; i < 2; ++i) {
             ptx::mbar_init(bar_q_full + 8 * i, 1);
             ptx::mbar_init(bar_q_copied + 8 * i, kNumVWarps);
@@ -753,6 +808,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     // phase always needs the waiter) and never runs ahead of it by more than one (every waiter goes through its
     // phases one by one).
 
+    // one of eight warps' share of Q's chunks in shared memory, BF16 to FP16 (element-wise, so the swizzled layout is untouched)
+    auto convert_q = [&](int w) {
+        constexpr int kVecs = L::kQChunks * kQChunkBytes / 16 / (kNumVWarps * 32);
+#pragma unroll 1
+        for (int i = 0; i < kVecs; ++i) {
+            const uint32_t at = q_base + uint32_t((i * kNumVWarps + w) * 32 + lane) * 16u;
+            ptx::sts_v4(at, bf16x8_to_f16x8(ptx::lds_v4(at)));
+        }
+    };
+
     if (warp >= kFirstKWarp && warp < kFirstVWarp) {
         // ───────────── K warps ─────────────
         // K rows 4 kw .. +3 of this block, all columns.  (Refilling the first half of the tile while the S MMAs still read the
@@ -761,15 +826,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         const int kw = warp - kFirstKWarp;
         const uint32_t piece = uint32_t(loader_piece(lane, R::kOwnRow));
         const LoaderAddr ad(4 * kw, piece, lane);
+        bool ok = true;
+        if (early_q) {
+            // (Q's chunks that stay in shared memory, before the first records are there)
+            ok = wait_for(bar_q_full, 0u, kStatusWaitQ, 2, 0);
+            if (ok) {
+                convert_q(kw);
+                ptx::fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) arrive_even(bar_q_ready);
+            }
+        }
 #pragma unroll 1
-        for (uint32_t g = 0;; ++g) {
+        for (uint32_t g = 0; ok; ++g) {
             const uint32_t st = g % kStages, raw = raw_base + st * R::kBytes;
             if (kw == 0 && lane == 0) trace_mark(a, 2, 8 * int(g));
             if (!wait_for(bar_raw_full + 8 * st, g / kStages, kStatusWaitRaw, 2, int(g))) break;
             const uint32_t meta = *reinterpret_cast<volatile uint32_t*>(&misc->meta[g % kTagRing]);
             if (!(meta & kMetaTile)) break;                              // the end of the stream
             const bool used = kw < tile_groups(meta_entries(meta));
-            bool ok = true;
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
                 uint4 x[2], rope;
@@ -814,43 +889,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         const LoaderAddr ad(16 * hr, piece, lane);
         const uint32_t v_span = v_base + 2u * uint32_t(jj) * kVChunkBytes + uint32_t(hb) * (kRowsPerBlock * 128u);
         uint32_t qn = 0;
+        // Q of an item has been sent for by the S warp (early: at once; else once the previous item's S MMAs had completed):
+        // chunks 0-5 reach tensor memory through a staging area in two rounds, the others land at their place in
+        // shared memory and are converted there.
+        auto set_up_q = [&](uint32_t g) -> bool {
 #pragma unroll 1
-        for (uint32_t g = 0;; ++g) {
+            for (int round = 0; round < 2; ++round) {
+                if (!wait_for(bar_q_full + 8 * round, qn, kStatusWaitQ, 2, int(g)) || (qn == 0u && !wait_tmem())) return false;
+                q_to_tmem<use_f16(SRC)>(round && qn == 0u ? v_base : q_stage, tmem + kTmemQ + 96 * round, vw, lane);
+                if (use_f16(SRC) && round == 0 && !early_q) convert_q(vw);
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar_q_copied + 8 * round);
+            }
+            ptx::tmem_wait_st();
+            ptx::tc_fence_before_sync();
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) arrive_even(bar_q_ready);
+            // (the first item's second round was staged in the V tile)
+            if (qn == 0u && !wait_for(bar_q_copied + 8, 0u, kStatusWaitQ, 2, int(g))) return false;
+            ++qn;
+            return true;
+        };
+        bool ok = !early_q || set_up_q(0u);
+#pragma unroll 1
+        for (uint32_t g = 0; ok; ++g) {
             const uint32_t st = g % kStages, raw = raw_base + st * R::kBytes;
             if (!wait_for(bar_raw_full + 8 * st, g / kStages, kStatusWaitRaw, 2, int(g))) break;
             const uint32_t meta = *reinterpret_cast<volatile uint32_t*>(&misc->meta[g % kTagRing]);
             if (!(meta & kMetaTile)) break;
-            if (meta & kMetaFirst) {
-                // Q of the item that starts here has been sent for by the S warp, once the previous item's S MMAs had completed:
-                // chunks 0-5 reach tensor memory through a staging area in two rounds, the others land at their place in
-                // shared memory and are converted there (element-wise, so the swizzled layout is untouched).
-                bool ok = true;
-#pragma unroll 1
-                for (int round = 0; round < 2 && ok; ++round) {
-                    ok = wait_for(bar_q_full + 8 * round, qn, kStatusWaitQ, 2, int(g)) && (qn > 0u || wait_tmem());
-                    if (!ok) break;
-                    q_to_tmem<use_f16(SRC)>(round && qn == 0u ? v_base : q_stage, tmem + kTmemQ + 96 * round, vw, lane);
-                    if (use_f16(SRC) && round == 0) {
-                        constexpr int kVecs = L::kQChunks * kQChunkBytes / 16 / (kNumVWarps * 32);
-#pragma unroll 1
-                        for (int i = 0; i < kVecs; ++i) {
-                            const uint32_t at = q_base + uint32_t((i * kNumVWarps + vw) * 32 + lane) * 16u;
-                            ptx::sts_v4(at, bf16x8_to_f16x8(ptx::lds_v4(at)));
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(bar_q_copied + 8 * round);
-                }
-                if (!ok) break;
-                ptx::tmem_wait_st();
-                ptx::tc_fence_before_sync();
-                ptx::fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) arrive_even(bar_q_ready);
-                // (the first item's second round was staged in the V tile)
-                if (qn == 0u && !wait_for(bar_q_copied + 8, 0u, kStatusWaitQ, 2, int(g))) break;
-                ++qn;
-            }
+            if (!early_q && (meta & kMetaFirst) && !set_up_q(g)) break;
             const int groups = tile_groups(meta_entries(meta)), rows = 16 * tile_ksteps(meta_entries(meta));
             const uint32_t valid = *reinterpret_cast<volatile uint32_t*>(&misc->mask[g % kTagRing][hb]);
             uint4 x[4], rope[is_ref_layout(SRC) ? 4 : 1];
@@ -902,6 +970,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     } else if (warp == kSWarp) {
         // ───────────── tensor-memory allocation, Q load, S = Q . K^T ─────────────
         constexpr uint32_t kDescHi = ptx::smem_desc_hi(1024);        // 8-row groups 1 KB apart
+        // Q rows of this block's 64 heads by TMA, one 64-column box per chunk, landing in the swizzled operand
+        // layout.  Rows past the end of Q read as zero; rows of a following request (H < 128) are computed
+        // but never written out.
+        auto q_row = [&](int n, int hg) { return n * a.H + hg * kHeadsPerCta + rank * kHeadsPerBlock; };
+        auto second_round = [&](uint32_t dst, int qrow0) {
+            ptx::mbar_arrive_expect_tx(bar_q_full + 8, kQStageChunks * kQChunkBytes);
+#pragma unroll
+            for (int c = 0; c < kQStageChunks; ++c) ptx::tma_load_2d(dst + uint32_t(c) * kQChunkBytes, &a.q_map, (kQStageChunks + c) * 64, qrow0, bar_q_full + 8);
+        };
+        auto send_for_q = [&](int qrow0, bool first) {
+            if (ptx::elect_one()) {
+                ptx::mbar_arrive_expect_tx(bar_q_full, uint32_t(kQStageChunks + L::kQChunks) * kQChunkBytes);
+#pragma unroll
+                for (int c = 0; c < kQStageChunks; ++c) ptx::tma_load_2d(q_stage + uint32_t(c) * kQChunkBytes, &a.q_map, c * 64, qrow0, bar_q_full);
+#pragma unroll
+                for (int c = 0; c < L::kQChunks; ++c) ptx::tma_load_2d(q_base + uint32_t(c) * kQChunkBytes, &a.q_map, (kQTmemChunks + c) * 64, qrow0, bar_q_full);
+                if (first) second_round(v_base, qrow0);                  // the V tile is still unused
+            }
+            __syncwarp();
+        };
+        // (the K and V warps wait for an early Q whether the row turns out empty or not)
+        if (early_q) send_for_q(q_row(blockIdx.y, blockIdx.x >> 1), true);
         ptx::tmem2_alloc(ptx::smem_u32(&misc->tmem_base), kTmemCols);
         ptx::tmem2_relinquish();
         ptx::tc_fence_before_sync();
@@ -918,27 +1008,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             if (ntiles > 0) {
                 // every S MMA of the previous item must have completed before its Q is replaced
                 if (gt > 0u && !wait_for(bar_s_full + 8 * ((gt - 1u) & 1u), (gt - 1u) >> 1, kStatusWaitSFull, 1, int(gt))) { ok = false;  break; }
-                // Q rows of this block's 64 heads by TMA, one 64-column box per chunk, landing in the swizzled operand
-                // layout.  Rows past the end of Q read as zero; rows of a following request (H < 128) are computed
-                // but never written out.
-                const int qrow0 = cur.n * a.H + cur.hg * kHeadsPerCta + rank * kHeadsPerBlock;
-                auto second_round = [&](uint32_t dst) {
-                    ptx::mbar_arrive_expect_tx(bar_q_full + 8, kQStageChunks * kQChunkBytes);
-#pragma unroll
-                    for (int c = 0; c < kQStageChunks; ++c) ptx::tma_load_2d(dst + uint32_t(c) * kQChunkBytes, &a.q_map, (kQStageChunks + c) * 64, qrow0, bar_q_full + 8);
-                };
-                if (ptx::elect_one()) {
-                    ptx::mbar_arrive_expect_tx(bar_q_full, uint32_t(kQStageChunks + L::kQChunks) * kQChunkBytes);
-#pragma unroll
-                    for (int c = 0; c < kQStageChunks; ++c) ptx::tma_load_2d(q_stage + uint32_t(c) * kQChunkBytes, &a.q_map, c * 64, qrow0, bar_q_full);
-#pragma unroll
-                    for (int c = 0; c < L::kQChunks; ++c) ptx::tma_load_2d(q_base + uint32_t(c) * kQChunkBytes, &a.q_map, (kQTmemChunks + c) * 64, qrow0, bar_q_full);
-                    if (qn == 0u) second_round(v_base);                  // the V tile is still unused
-                }
-                __syncwarp();
+                const int qrow0 = q_row(cur.n, cur.hg);
+                if (!early_q) send_for_q(qrow0, qn == 0u);
                 if (qn > 0u) {
                     if (!wait_for(bar_q_copied, qn, kStatusWaitQ, 1, int(gt))) { ok = false;  break; }
-                    if (ptx::elect_one()) second_round(q_stage);
+                    if (ptx::elect_one()) second_round(q_stage, qrow0);
                     __syncwarp();
                 }
                 if (rank == 0) {
@@ -1097,7 +1171,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(bar_id_full + bars);
             if (!(cur.meta & kMetaTile)) break;                          // that was the end mark
-            if (p == 0 && (c0.meta & kMetaFirst)) prefetch_q_l2<NCHUNK>(a, c0.n, c0.hg, rank, lane);
+            if (!early_q && p == 0 && (c0.meta & kMetaFirst)) prefetch_q_l2<NCHUNK>(a, c0.n, c0.hg, rank, lane);
         }
         __syncwarp();
     } else if (warp >= kFetchWarp) {

@@ -323,6 +323,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const void* tenso
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const void* tensor_map, int x, int y, int z, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        :
+        : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(tensor_map)), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
+
 // Four rows of a row-major tensor named by their numbers (tile::gather4; the map's box is one row high), laid down one
 // after the other at smem_dst, which is a multiple of 128 bytes.
 __device__ __forceinline__ void tma_gather4(uint32_t smem_dst, const void* tensor_map, int x, const int4& rows, uint32_t bar) {
@@ -378,6 +386,7 @@ __device__ __forceinline__ uint4 ldg_nc_v4(const void* p) {
     return v;
 }
 
+__device__ __forceinline__ void prefetch_tensormap(const void* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }

@@ -53,3 +53,31 @@ def test_row_lengths_at_tile_edges(lib, n):
                              gu.dev(case.Kswa_s), gu.dev(case.Kswa_rope, torch.bfloat16), gu.dev(case.sink), case.sm_scale, M_cur=n, swa_len=max(win, 1))
     torch.cuda.synchronize()
     gu.check_out(gu.out_to_f32(got), want[0] if isinstance(want, tuple) else want, f"planes n={n}")
+
+
+class _PagesInOrder:
+    """Stands in for the generator that shuffles pages: page numbers follow one another."""
+    def __init__(self, seed):
+        self.integers = np.random.default_rng(seed).integers
+
+    def permutation(self, n):
+        return np.arange(n)
+
+
+@pytest.mark.parametrize("page", [16, 32, 64])
+@pytest.mark.parametrize("m_cur", [0, 1, 62, 66, 131])
+def test_packed_pages_fetched_four_tokens_at_a_time(lib, page, m_cur):
+    """A group of four rows is fetched as one box only inside a page: window rows that are not aligned to four cross page borders,
+    here also into the page that lies next in memory."""
+    case = orc.make_ref_layout_case(seed=1000 + m_cur, B=2, H=16, M_cur=140, swa_len=128)
+    kv, bt = orc.pack_ref_pages(case.Kc, case.Kc_s, case.Kc_rope, page, _PagesInOrder(1))
+    sw, sbt = orc.pack_ref_pages(case.Kswa, case.Kswa_s, case.Kswa_rope, page, _PagesInOrder(2))
+    m, w = np.array([m_cur, m_cur + 1], np.int32), np.array([128, 67], np.int32)
+    st = lib.new_status("cuda")
+    out, lse = lib.hca_packed_decode(gu.dev(case.Q, torch.bfloat16), gu.dev(kv), gu.dev(bt), gu.dev(m), gu.dev(sw), gu.dev(sbt), gu.dev(w),
+                                     case.sm_scale, page_size=page, attn_sink=gu.dev(case.sink), num_splits=1, status=st)
+    torch.cuda.synchronize()
+    assert st.cpu().tolist() == [0, 0, 0, 0]
+    want, want_lse = orc.hca_decode_packed_pages(case.Q, kv, bt, m, sw, sbt, w, case.sink, case.sm_scale, page)
+    gu.check_out(gu.out_to_f32(out), want, f"page={page} m_cur={m_cur}")
+    gu.check_lse(lse.cpu().numpy(), want_lse, f"page={page} m_cur={m_cur}")
