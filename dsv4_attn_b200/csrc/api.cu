@@ -594,9 +594,10 @@ extern "C" int dsv4_attn_plan_splits(int rows, int H, int max_len, int num_sms) 
     const int64_t units = int64_t(rows) * 2 * ((H + kHeadsPerCta - 1) / kHeadsPerCta);
     // Cost model in units of one tile's time: a block costs a fixed set-up (Q
     // load, tensor-memory allocation, epilogue) plus its tiles; blocks run in
-    // waves of `num_sms`; splitting adds the partial write + merge read.
-    // constants fitted to measurements on B200 (split sweep at 512 units x 32 tiles)
-    const double fixed = 4.0, merge_per_split = 1.8, merge_launch = 2.0;
+    // waves of `num_sms`; splitting adds the partial write + merge read, and the merge of one row takes its splits in turn.
+    // constants fitted to measurements on B200 (split sweeps, 1 to 100 rows x 2 to 64 tiles: within 4 % of the best split count;
+    // a set-up of 4 tiles cut 48 rows of 32 tiles in three, 59 us against 55, and one such row in 32, 23 us against 19)
+    const double fixed = 7.0, merge_per_split = 1.8, merge_launch = 2.0, merge_serial = 0.2;
     double best = 1e300;
     int best_s = 1;
     const int max_s = tiles < DSV4_MAX_SPLITS ? tiles : DSV4_MAX_SPLITS;
@@ -606,7 +607,7 @@ extern "C" int dsv4_attn_plan_splits(int rows, int H, int max_len, int num_sms) 
         const int64_t blocks = units * s;
         const double waves = std::ceil(double(blocks) / num_sms);
         double cost = waves * (fixed + tps);
-        if (s > 1) cost += merge_per_split * s * (double(units) / num_sms) + merge_launch;   // partials written and re-read, one more launch
+        if (s > 1) cost += merge_per_split * s * (double(units) / num_sms) + merge_launch + merge_serial * s;   // partials written and re-read, one more launch
         if (cost < best - 1e-9) { best = cost;  best_s = s; }
     }
     return best_s;
