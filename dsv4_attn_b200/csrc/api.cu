@@ -263,11 +263,11 @@ cudaError_t launch_simt(const DecodeArgs& a, int rows, int max_tok, cudaStream_t
 }
 
 cudaError_t launch_combine(const CombineArgs& c, cudaStream_t stream) {
-    if (c.unit_nsplits != nullptr) {      // resident blocks (four per SM) share out what the plan cut, but no more than could have work
-        const int64_t most = int64_t(c.N) * c.hgs * ((c.H < 128 ? c.H : 128) + kCombineWarps - 1) / kCombineWarps;
-        const int64_t resident = int64_t(device_sms()) * 4;
-        return launch(combine_sched_kernel, dim3(unsigned(most < resident ? most : resident)), kCombineWarps * 32, 0, stream, c);
-    }
+    // A scheduled batch whose (row, head) warps would not all be resident at once (four blocks per SM): resident blocks share out what the
+    // plan cut.  Below that a warp looks its unit up and is done sooner than a block has gathered the cut units.
+    const int64_t resident = int64_t(device_sms()) * 4;
+    if (c.unit_nsplits != nullptr && int64_t(c.N) * c.H > resident * kCombineWarps)
+        return launch(combine_sched_kernel, dim3(unsigned(resident)), kCombineWarps * 32, 0, stream, c);
     const int64_t units = int64_t(c.N) * c.H;
     return launch(combine_kernel, dim3(unsigned((units + kCombineWarps - 1) / kCombineWarps)), kCombineWarps * 32, 0, stream, c);
 }
@@ -828,16 +828,13 @@ extern "C" int dsv4_rope_norm_fwd(const Dsv4RopeNormParams* p, void* stream) {
         known_theta = a.theta;
     }
     std::memcpy(a.freq, known_freq, sizeof(known_freq));
-    // Vectors of a row per warp: as many as still leave every SM eight warps, the number that hides a load's latency
-    // (a larger group computes the angles once for more vectors and keeps more loads in flight per warp).
+    // Two vectors of a row per warp where that still leaves every SM eight warps, the number that hides a load's latency.
     const int64_t fill = int64_t(device_sms()) * 8;
-    int group = 1;
-    if (a.vecs_per_row >= 4 && a.n_rows * ((a.vecs_per_row + 3) / 4) >= fill) group = 4;
-    else if (a.vecs_per_row >= 2 && a.n_rows * ((a.vecs_per_row + 1) / 2) >= fill) group = 2;
+    const int group = a.vecs_per_row >= 2 && a.n_rows * ((a.vecs_per_row + 1) / 2) >= fill ? 2 : 1;
     const int64_t items = a.n_rows * ((a.vecs_per_row + group - 1) / group);
     const int64_t want = (items + kRopeNormThreads / 32 - 1) / (kRopeNormThreads / 32);
     const int64_t cap = fill;
-    auto kernel = group == 4 ? rope_norm_kernel<4> : (group == 2 ? rope_norm_kernel<2> : rope_norm_kernel<1>);
+    auto kernel = group == 2 ? rope_norm_kernel<2> : rope_norm_kernel<1>;
     return int(launch(kernel, dim3(unsigned(want < cap ? want : cap)), kRopeNormThreads, 0, static_cast<cudaStream_t>(stream), a));
 }
 
@@ -890,6 +887,7 @@ extern "C" int dsv4_indexer_topk_fwd(const Dsv4IndexerTopkParams* p, void* strea
     a.tiles_per_cta = (tiles_cap + ctas - 1) / ctas;
     const int grid_x = (tiles_cap + a.tiles_per_cta - 1) / a.tiles_per_cta;
     a.B = p->B;  a.s_q = p->s_q;  a.max_pages = p->max_pages;  a.num_pages = p->num_pages;
+    a.q = static_cast<const uint8_t*>(p->q_fp8);
     a.q_weight = p->q_weight;  a.block_table = p->block_table;  a.n_vis = p->n_vis;
     a.scores = p->scores;  a.score_stride = p->score_stride;  a.status = p->status;
     a.wait_ns = g_wait_ns.load(std::memory_order_relaxed);

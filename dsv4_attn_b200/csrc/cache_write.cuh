@@ -40,7 +40,7 @@ struct CacheDest {
 // outside the block table or the table names a page outside the pool.
 __device__ __forceinline__ uint8_t* entry_address(const CacheDest& d, int b, int64_t e) {
     if (e >= 0 && (e >> 6) < d.max_pages) {
-        const int page = __ldg(d.block_table + int64_t(b) * d.max_pages + (e >> 6));
+        const int page = ptx::ld(d.block_table + int64_t(b) * d.max_pages + (e >> 6));
         if (page >= 0 && page < d.num_pages) return d.kv_pool + (int64_t(page) * 64 + (e & 63)) * 656;
     }
     if (d.status != nullptr && atomicCAS(d.status, 0, kStatusBadInsert) == 0) {
@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
 #pragma unroll
             for (int j = 0; j < kHcaBatch; ++j) {
                 if (FULL || r + j < r1) {
-                    zv[j] = ptx::ldg_nc_v4(a.Z + base + int64_t(r + j) * a.stride_n);
-                    cv[j] = ptx::ldg_nc_v4(a.C + base + int64_t(r + j) * a.stride_n);
-                    bv[j] = __ldg(reinterpret_cast<const uint4*>(a.bias + int64_t(r + j) * a.c + ch));
+                    zv[j] = ptx::ldg_stream_v4(a.Z + base + int64_t(r + j) * a.stride_n);
+                    cv[j] = ptx::ldg_stream_v4(a.C + base + int64_t(r + j) * a.stride_n);
+                    bv[j] = ptx::ld(reinterpret_cast<const uint4*>(a.bias + int64_t(r + j) * a.c + ch));
                 }
             }
             // The reference maximum of the step is found in packed BF16 arithmetic (one add and
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
     if (a.dst.kv_pool == nullptr) return;
     // cache insert (c == 576, one slab): threads 0..63 hold the latent, 64..71 the RoPE tail
     uint8_t* entry = nullptr;
-    if ((t & 31) == 0 || t >= 64) entry = entry_address(a.dst, b, int64_t(__ldg(a.dst.insert_pos + b)) + blk);
+    if ((t & 31) == 0 || t >= 64) entry = entry_address(a.dst, b, int64_t(ptx::ld(a.dst.insert_pos + b)) + blk);
     if (t < 64) {
         entry = reinterpret_cast<uint8_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(entry), 0));
         float amax = 0.f;
@@ -264,13 +264,13 @@ __global__ void __launch_bounds__(kInsertThreads) kv_quantize_insert_kernel(cons
     for (int64_t row = int64_t(blockIdx.x) * (kInsertThreads / 32) + (threadIdx.x >> 5); row < total;
          row += int64_t(gridDim.x) * (kInsertThreads / 32)) {
         const int b = int(row / a.T), t = int(row % a.T);
-        if (a.n_rows != nullptr && t >= __ldg(a.n_rows + b)) continue;
+        if (a.n_rows != nullptr && t >= ptx::ld(a.n_rows + b)) continue;
         const __nv_bfloat16* src = a.rows + int64_t(b) * a.stride_b + int64_t(t) * a.stride_t;
-        const uint4 x0 = ptx::ldg_nc_v4(src + 16 * lane);
-        const uint4 x1 = ptx::ldg_nc_v4(src + 16 * lane + 8);
-        const uint32_t rope = __ldg(reinterpret_cast<const uint32_t*>(src + 512 + 2 * lane));
+        const uint4 x0 = ptx::ldg_stream_v4(src + 16 * lane);
+        const uint4 x1 = ptx::ldg_stream_v4(src + 16 * lane + 8);
+        const uint32_t rope = ptx::ld(reinterpret_cast<const uint32_t*>(src + 512 + 2 * lane));
         uint8_t* entry = nullptr;
-        if (lane == 0) entry = entry_address(a.dst, b, int64_t(__ldg(a.dst.insert_pos + b)) + t);
+        if (lane == 0) entry = entry_address(a.dst, b, int64_t(ptx::ld(a.dst.insert_pos + b)) + t);
         entry = reinterpret_cast<uint8_t*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(entry), 0));
         float f[16];
         {

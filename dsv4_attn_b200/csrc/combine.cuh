@@ -53,14 +53,14 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
                                            int64_t po_off, int64_t po_stride) {
     // pass 1: maximum and sum over splits.  The first 32 LSEs are loaded once (one per lane) and serve the maximum,
     // the sum and the weights; only rows with more than 32 splits go back to memory.
-    const float l_first = (lane < S) ? __ldg(pl + int64_t(lane) * pl_stride) : -CUDART_INF_F;
+    const float l_first = (lane < S) ? ptx::ld(pl + int64_t(lane) * pl_stride) : -CUDART_INF_F;
     float mx = l_first;
-    for (int s = lane + 32; s < S; s += 32) mx = fmaxf(mx, __ldg(pl + int64_t(s) * pl_stride));
+    for (int s = lane + 32; s < S; s += 32) mx = fmaxf(mx, ptx::ld(pl + int64_t(s) * pl_stride));
     mx = warp_max(mx);
     float sum = 0.f;
     if (mx != -CUDART_INF_F) {
         sum = exp2f(l_first - mx);
-        for (int s = lane + 32; s < S; s += 32) sum += exp2f(__ldg(pl + int64_t(s) * pl_stride) - mx);
+        for (int s = lane + 32; s < S; s += 32) sum += exp2f(ptx::ld(pl + int64_t(s) * pl_stride) - mx);
     }
     sum = warp_sum(sum);
     const bool has = sum != 0.f;
@@ -69,7 +69,7 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
         a.lse[int64_t(n) * a.stride_lse_n + h] = has ? glse * 0.6931471805599453f : -CUDART_INF_F;
     float denom = glse;
     if (a.attn_sink != nullptr) {
-        const float s2 = __ldg(a.attn_sink + h) * 1.4426950408889634f;
+        const float s2 = ptx::ld(a.attn_sink + h) * 1.4426950408889634f;
         denom = has ? glse + log2f(1.f + exp2f(s2 - glse)) : s2;
     }
 
@@ -83,7 +83,7 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
         // each lane computes the weight of one split of this group; broadcast by shuffle
         float w_mine = 0.f;
         if (s0 + lane < S) {
-            const float l = (s0 == 0) ? l_first : __ldg(pl + int64_t(s0 + lane) * pl_stride);
+            const float l = (s0 == 0) ? l_first : ptx::ld(pl + int64_t(s0 + lane) * pl_stride);
             w_mine = (l == -CUDART_INF_F || denom == -CUDART_INF_F) ? 0.f : exp2f(l - denom);
         }
         const int cnt = min(32, S - s0);
@@ -102,7 +102,7 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
                 for (int j = 0; j < 2; ++j)
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
-                        v[j][i] = __ldg(reinterpret_cast<const uint4*>(sb + int64_t(k0 + j < cnt ? j : 0) * po_stride + i * 256));
+                        v[j][i] = ptx::ld(reinterpret_cast<const uint4*>(sb + int64_t(k0 + j < cnt ? j : 0) * po_stride + i * 256));
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -125,8 +125,8 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
                         // not predicated on the weight: the loads go out before the weights are known; what an
                         // empty split's slot holds is discarded below
                         const float4* q = reinterpret_cast<const float4*>(src + int64_t(k0 + j < cnt ? j : 0) * po_stride + i * 256);
-                        v[j][2 * i] = __ldg(q);
-                        v[j][2 * i + 1] = __ldg(q + 1);
+                        v[j][2 * i] = ptx::ld(q);
+                        v[j][2 * i + 1] = ptx::ld(q + 1);
                     }
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
@@ -155,19 +155,36 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
     }
 }
 
-// Every (row, head) has num_splits partials.
-__global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __grid_constant__ CombineArgs a) {
+// One warp per (row, head) of the batch: every one has num_splits partials, or those the plan says.
+__global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const CombineArgs a) {
     ptx::pdl_trigger();
     ptx::pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t unit = int64_t(blockIdx.x) * kCombineWarps + warp;   // (row, head) flattened
     if (unit >= int64_t(a.N) * a.H) return;
     const int n = int(unit / a.H), h = int(unit % a.H);
-    merge_head(a, n, h, lane, a.num_splits, a.partial_lse + int64_t(n) * a.stride_pl_n + h, a.stride_pl_split,
-               int64_t(n) * a.stride_po_n + int64_t(h) * a.stride_po_h + lane * 8, a.stride_po_split);
+    int S = a.num_splits;
+    const float* pl;
+    int64_t pl_stride, po_off, po_stride;      // po_*: element offsets into partial_o (FP32 or BF16 elements)
+    if (a.unit_nsplits != nullptr) {
+        const int u = n * a.hgs + (h >> 7);
+        S = ptx::ld(a.unit_nsplits + u);
+        if (S <= 1) return;
+        const int64_t row = int64_t(ptx::ld(a.unit_slot + u)) * 128 + (h & 127);
+        pl = a.partial_lse + row;
+        pl_stride = 128;
+        po_off = row * 512 + lane * 8;
+        po_stride = 128 * 512;
+    } else {
+        pl = a.partial_lse + int64_t(n) * a.stride_pl_n + h;
+        pl_stride = a.stride_pl_split;
+        po_off = int64_t(n) * a.stride_po_n + int64_t(h) * a.stride_po_h + lane * 8;
+        po_stride = a.stride_po_split;
+    }
+    merge_head(a, n, h, lane, S, pl, pl_stride, po_off, po_stride);
 }
 
-// After a scheduled decode.  A plan cuts at most as many units as there are block pairs, usually far fewer than the batch has, so
+// After a scheduled decode of a large batch.  A plan cuts at most as many units as there are block pairs, usually far fewer than the batch has, so
 // the grid is what is resident at once and its blocks share the cut units out, eight heads at a time: each block gathers them from
 // the plan's list (256 requests, mixed lengths: 12.5 -> 10 us cold against one warp per (row, head) of the batch, of which nine in ten had nothing to do).
 __global__ void __launch_bounds__(kCombineWarps * 32) combine_sched_kernel(const __grid_constant__ CombineArgs a) {
@@ -186,7 +203,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_sched_kernel(const
 #pragma unroll
         for (int i = 0; i < kPerThread; ++i) {
             const int u = base + (warp * kPerThread + i) * 32 + lane;
-            cut[i] = __ballot_sync(0xFFFFFFFFu, u < n_units && __ldg(a.unit_nsplits + u) > 1);
+            cut[i] = __ballot_sync(0xFFFFFFFFu, u < n_units && ptx::ld(a.unit_nsplits + u) > 1);
             mine += __popc(cut[i]);
         }
         __syncthreads();                      // the chunk before is done with the list
@@ -212,8 +229,8 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_sched_kernel(const
             const int u = s_unit[j / slices], n = u / a.hgs;
             const int in_group = int(j % slices) * kCombineWarps + warp, h = (u % a.hgs) * 128 + in_group;
             if (h >= a.H) continue;
-            const int64_t row = int64_t(__ldg(a.unit_slot + u)) * 128 + in_group;
-            merge_head(a, n, h, lane, __ldg(a.unit_nsplits + u), a.partial_lse + row, 128, row * 512 + lane * 8, 128 * 512);
+            const int64_t row = int64_t(ptx::ld(a.unit_slot + u)) * 128 + in_group;
+            merge_head(a, n, h, lane, ptx::ld(a.unit_nsplits + u), a.partial_lse + row, 128, row * 512 + lane * 8, 128 * 512);
         }
         job0 += jobs;
     }

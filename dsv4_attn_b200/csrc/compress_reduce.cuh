@@ -44,14 +44,14 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
 template <int VEC> struct BfVec;
 template <> struct BfVec<8> {
     using T = uint4;
-    static __device__ __forceinline__ T load_stream(const __nv_bfloat16* p) { return ptx::ldg_nc_v4(p); }
+    static __device__ __forceinline__ T load_stream(const __nv_bfloat16* p) { return ptx::ldg_stream_v4(p); }
     static __device__ __forceinline__ void unpack(const T& v, float (&f)[8]) { unpack8(v, f); }
 };
 template <> struct BfVec<4> {
     using T = uint2;
     static __device__ __forceinline__ T load_stream(const __nv_bfloat16* p) {
         T v;
-        asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+        asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
         return v;
     }
     static __device__ __forceinline__ void unpack(const T& v, float (&f)[4]) {
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
                     cb[j] = BfVec<VEC>::load_stream(a.C_b + row_b + j * a.stride_c_n);
                 }
             }
-            auto bias = [&](int j, bool bside) { return __ldg(reinterpret_cast<const V*>((bside ? a.B_b : a.B_a) + int64_t(j) * a.c_out + ch)); };
+            auto bias = [&](int j, bool bside) { return ptx::ld(reinterpret_cast<const V*>((bside ? a.B_b : a.B_a) + int64_t(j) * a.c_out + ch)); };
             // The reference maximum is found in packed BF16 arithmetic: any value close to the true maximum serves, as long as the
             // same one is used for every weight.  The logits themselves are formed in FP32, two channels an instruction.
             constexpr int P = VEC / 2;

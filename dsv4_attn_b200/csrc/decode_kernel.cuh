@@ -341,7 +341,7 @@ constexpr int kNoPage = -2;
 // Stage 1 (CSA only): the index-list value of entry `ent` of the tile, -1 where there is none.
 __device__ __forceinline__ int resolve_index(const DecodeArgs& a, const TileCtx& c, int ent) {
     const int v = c.v0 + ent;
-    if ((c.meta & kMetaTile) && v < c.n_tok) return __ldg(a.indices + int64_t(c.n) * a.topk + v);
+    if ((c.meta & kMetaTile) && v < c.n_tok) return ptx::ld(a.indices + int64_t(c.n) * a.topk + v);
     return -1;
 }
 
@@ -356,7 +356,7 @@ __device__ __forceinline__ PendingId resolve_issue(const DecodeArgs& a, const Ti
     if constexpr (SRC == kSrcCsa) {
         if (e >= 0 && e < c.kv_len_n) {
             if ((e >> 6) < a.max_pages) {
-                p.page = __ldg(a.block_table + int64_t(c.b) * a.max_pages + (e >> 6));
+                p.page = ptx::ld(a.block_table + int64_t(c.b) * a.max_pages + (e >> 6));
                 p.id = kIdValid | uint32_t(e & 63);
             } else {
                 report_status(a.status, kStatusBadIndex, 4, e);
@@ -366,7 +366,7 @@ __device__ __forceinline__ PendingId resolve_issue(const DecodeArgs& a, const Ti
         if (in_row) {
             if (v < c.kv_len_n) {
                 if ((v >> 6) < a.max_pages) {
-                    p.page = __ldg(a.block_table + int64_t(c.b) * a.max_pages + (v >> 6));
+                    p.page = ptx::ld(a.block_table + int64_t(c.b) * a.max_pages + (v >> 6));
                     p.id = kIdValid | uint32_t(v & 63);
                 } else {
                     report_status(a.status, kStatusBadIndex, 4, v);
@@ -388,7 +388,7 @@ __device__ __forceinline__ PendingId resolve_issue(const DecodeArgs& a, const Ti
             const int32_t* table = swa ? a.pg_swa_table : a.block_table;
             const int cols = swa ? a.pg_swa_max_pages : a.max_pages;
             if (pool != nullptr && (w >> a.pg_page_shift) < cols) {
-                p.page = __ldg(table + int64_t(c.b) * cols + (w >> a.pg_page_shift));
+                p.page = ptx::ld(table + int64_t(c.b) * cols + (w >> a.pg_page_shift));
                 p.id = kIdValid | (swa ? kIdSecond : 0u) | uint32_t(w & slot_mask);
             }
         }
@@ -461,12 +461,12 @@ __device__ __forceinline__ void prefetch_start(const DecodeArgs& a, int n, int h
 template <int SRC>
 __device__ __forceinline__ void row_lengths(const DecodeArgs& a, int n, int& n_tok, int& kv_len_n) {
     if constexpr (SRC == kSrcCsa) {
-        const int raw = (a.topk_len != nullptr) ? __ldg(a.topk_len + n) : a.topk;
+        const int raw = (a.topk_len != nullptr) ? ptx::ld(a.topk_len + n) : a.topk;
         n_tok = min(max(raw, 0), a.topk);
-        kv_len_n = (a.kv_len != nullptr) ? __ldg(a.kv_len + n) : 0x7FFFFFFF;
+        kv_len_n = (a.kv_len != nullptr) ? ptx::ld(a.kv_len + n) : 0x7FFFFFFF;
     } else if constexpr (SRC == kSrcHca || SRC == kSrcRefPaged) {
-        kv_len_n = max(__ldg(a.kv_len + n), 0);
-        n_tok = kv_len_n + max(__ldg(a.win_len + n), 0);
+        kv_len_n = max(ptx::ld(a.kv_len + n), 0);
+        n_tok = kv_len_n + max(ptx::ld(a.win_len + n), 0);
     } else {
         kv_len_n = a.ref_m_cur;
         n_tok = a.ref_m_cur + a.ref_swa_len;
@@ -507,12 +507,12 @@ __device__ __forceinline__ uint2 load_ref_scales(const DecodeArgs& a, uint32_t i
     if (id & kIdValid) {
         const RecordPtr<SRC> p(a, id);
         if constexpr (SRC == kSrcRefPaged) {
-            w = __ldg(reinterpret_cast<const uint2*>(p.scale));
+            w = ptx::ld(reinterpret_cast<const uint2*>(p.scale));
         } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w.x |= uint32_t(__ldg(p.scale + i)) << (8 * i);
+            for (int i = 0; i < 4; ++i) w.x |= uint32_t(ptx::ld(p.scale + i)) << (8 * i);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) w.y |= uint32_t(__ldg(p.scale + 4 + i)) << (8 * i);
+            for (int i = 0; i < 3; ++i) w.y |= uint32_t(ptx::ld(p.scale + 4 + i)) << (8 * i);
         }
     }
     return w;
@@ -710,7 +710,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         Item it;
         if (sched) {
             const int4* rec = reinterpret_cast<const int4*>(a.sched_items + int64_t(item_begin + k) * kItemWords);
-            const int4 r0 = __ldg(rec), r1 = __ldg(rec + 1);
+            const int4 r0 = ptx::ld(rec), r1 = ptx::ld(rec + 1);
             it.n = r0.x;  it.hg = r0.y;  it.tile0 = r0.z;  it.ntiles = r0.w;
             it.slot = r1.x;  it.n_tok = r1.y;  it.kv_len_n = r1.z;
         } else {
@@ -784,8 +784,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     ptx::pdl_wait();
     if (sched) {
         const int pair = blockIdx.x >> 1;
-        item_begin = __ldg(a.sched_pair_begin + pair);
-        n_items = __ldg(a.sched_pair_begin + pair + 1) - item_begin;
+        item_begin = ptx::ld(a.sched_pair_begin + pair);
+        n_items = ptx::ld(a.sched_pair_begin + pair + 1) - item_begin;
     }
     // All 512 columns are allocated, so tensor memory starts at address 0 (checked where it is allocated): as a constant it keeps the
     // operands of every tcgen05 instruction out of vector registers.
@@ -1343,7 +1343,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             if (tid == 0 && k == n_items - 1 && (sched || a.num_splits > 1)) ptx::pdl_trigger();
             float denom = l_sum;
             if (final_out && a.attn_sink != nullptr && write) {
-                const float s2 = __ldg(a.attn_sink + h0 + r) * 1.4426950408889634f;
+                const float s2 = ptx::ld(a.attn_sink + h0 + r) * 1.4426950408889634f;
                 denom = (l_sum > 0.f) ? l_sum + ptx::ex2(s2 - m_ref) : 1.f;   // empty row: O is 0 anyway
             }
             const float inv = (l_sum > 0.f) ? 1.f / denom : 0.f;

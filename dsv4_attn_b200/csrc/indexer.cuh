@@ -47,6 +47,7 @@ struct IndexerArgs {
     alignas(64) CUtensorMap q_map;       // q as [B*s_q*64, 128] bytes, box s_q*64 rows, 128-byte swizzle
     int B, s_q, max_pages, tiles_per_cta;
     int64_t num_pages;
+    const uint8_t* q;                    // [B, s_q, 64, 128] e4m3
     const float* q_weight;               // [B, s_q, 64]
     const int32_t* block_table;          // [B, max_pages]
     const int32_t* n_vis;                // [B, s_q]
@@ -104,9 +105,19 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
     const int b = blockIdx.y;
     const int N = a.s_q * kIdxHeads;
 
+    // The chain lengths -> block table -> key pages meets DRAM once instead of three times: what the block will read first is pulled into L2 before
+    // the wait on the previous kernel (nothing is read here).
+    {
+        const int64_t first = int64_t(blockIdx.x) * a.tiles_per_cta * 2;
+        const uint8_t* q = a.q + int64_t(b) * N * kIdxDim;
+        if (tid < N) ptx::prefetch_l2(q + int64_t(tid) * kIdxDim);
+        else if (tid == 160) ptx::prefetch_l2(a.n_vis + b * a.s_q);
+        else if (tid == 161 && first < a.max_pages) ptx::prefetch_l2(a.block_table + int64_t(b) * a.max_pages + first);
+        else if (tid >= 164 && tid < 164 + N / 32) ptx::prefetch_l2(a.q_weight + int64_t(b) * N + (tid - 164) * 32);
+    }
     ptx::pdl_wait();
     int vis_max = 0;
-    for (int t = 0; t < a.s_q; ++t) vis_max = max(vis_max, __ldg(a.n_vis + b * a.s_q + t));
+    for (int t = 0; t < a.s_q; ++t) vis_max = max(vis_max, ptx::ld(a.n_vis + b * a.s_q + t));
     vis_max = min(vis_max, a.max_pages * kIdxPageKeys);
     const int tiles_total = (vis_max + kIdxTileKeys - 1) / kIdxTileKeys;
     const int tile0 = min(int(blockIdx.x) * a.tiles_per_cta, tiles_total);
@@ -124,7 +135,7 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
         ptx::mbar_init(bar_q, 1);
         ptx::fence_mbar_init();
     }
-    if (tid < N) sm->weight[tid] = __ldg(a.q_weight + int64_t(b) * N + tid);
+    if (tid < N) sm->weight[tid] = ptx::ld(a.q_weight + int64_t(b) * N + tid);
     if (warp == 1) {
         ptx::tmem_alloc(ptx::smem_u32(&sm->tmem_base), kIdxTmemCols);
         ptx::tmem_relinquish();
@@ -140,23 +151,31 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
         if (lane == 0) {
             ptx::mbar_arrive_expect_tx(bar_q, uint32_t(N) * kIdxDim);
             ptx::tma_load_2d(q_smem, &a.q_map, 0, b * N, bar_q);
-            const int pages_vis = (vis_max + kIdxPageKeys - 1) / kIdxPageKeys;
-            for (int i = 0; i < ntiles && ok; ++i) {
-                const int st = i % kIdxStages;
-                if (i >= kIdxStages && !ptx::mbar_wait(bar_empty + 8 * st, uint32_t(i / kIdxStages - 1) & 1u, a.wait_ns)) {
-                    report_status(a.status, kStatusWaitIndexer, 0, tile0 + i);
-                    ok = false;
-                    break;
-                }
-                int page[2];
+        }
+        const int pages_vis = (vis_max + kIdxPageKeys - 1) / kIdxPageKeys;
+        // the lanes hold the page numbers of 16 tiles, those of the next 16 are on their way
+        auto load_pages = [&](int i) -> int {
+            const int lp = 2 * (tile0 + i) + lane;                      // logical page of the request
+            return (lp < pages_vis) ? ptx::ld(a.block_table + int64_t(b) * a.max_pages + lp) : -1;
+        };
+        int cur = -1, ahead = load_pages(0);
+        for (int i = 0; i < ntiles; ++i) {
+            const int st = i % kIdxStages;
+            if (i % 16 == 0) { cur = ahead;  ahead = load_pages(i + 16); }
+            const int page[2] = {__shfl_sync(0xFFFFFFFFu, cur, 2 * (i % 16)), __shfl_sync(0xFFFFFFFFu, cur, 2 * (i % 16) + 1)};
+            const bool w = i < kIdxStages || ptx::mbar_wait(bar_empty + 8 * st, uint32_t(i / kIdxStages - 1) & 1u, a.wait_ns);
+            if (!__all_sync(0xFFFFFFFFu, w)) {
+                report_status(a.status, kStatusWaitIndexer, 0, tile0 + i);
+                break;
+            }
+            if (lane == 0) {
                 uint32_t okmask = 0, bytes = 0;
-                for (int j = 0; j < 2; ++j) {
-                    const int lp = 2 * (tile0 + i) + j;            // logical page of the request
-                    page[j] = (lp < pages_vis) ? __ldg(a.block_table + int64_t(b) * a.max_pages + lp) : -1;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
                     if (page[j] >= 0 && page[j] < a.num_pages) { okmask |= 1u << j;  bytes += kIdxPageKeys * kIdxDim + 256; }
-                }
                 sm->page_ok[st] = okmask;
                 ptx::mbar_arrive_expect_tx(bar_full + 8 * st, bytes);
+#pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     if (!((okmask >> j) & 1u)) continue;
                     ptx::tma_load_2d(key_smem + st * kIdxStageKeyBytes + j * (kIdxPageKeys * kIdxDim), &a.key_map, 0,
@@ -165,6 +184,7 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
                                      page[j] * kIdxPageRows + kIdxPageKeys, bar_full + 8 * st);
                 }
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ───────────── MMA issue: S^T[128 keys x N] = K[128 x 128] . Q[N x 128]^T, four K steps of 32 ─────────────
@@ -196,8 +216,8 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
         const int r = quarter * 32 + lane;                             // key row inside the tile
         const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
         int vis[2];
-        vis[0] = min(__ldg(a.n_vis + b * a.s_q), a.max_pages * kIdxPageKeys);
-        vis[1] = (a.s_q > 1) ? min(__ldg(a.n_vis + b * a.s_q + 1), a.max_pages * kIdxPageKeys) : 0;
+        vis[0] = min(ptx::ld(a.n_vis + b * a.s_q), a.max_pages * kIdxPageKeys);
+        vis[1] = (a.s_q > 1) ? min(ptx::ld(a.n_vis + b * a.s_q + 1), a.max_pages * kIdxPageKeys) : 0;
         for (int i = 0; i < ntiles && ok; ++i) {
             const int st = i % kIdxStages, d = i & 1;
             const bool w = ptx::mbar_wait(bar_acc_full + 8 * d, uint32_t(i / 2) & 1u, a.wait_ns) &&
@@ -249,6 +269,7 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
 constexpr int kTopkThreads = 1024;
 constexpr int kTopkBins = 1024;          // one bin per thread in the suffix scan
 constexpr int kTopkCand = 4096;          // candidates of the threshold bin kept in shared memory
+constexpr int kTopkRanked = 384;         // up to this many are ranked by comparison (at 384 about as long as the radix select)
 
 // order-preserving map float -> uint32 (larger float = larger key)
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -359,7 +380,7 @@ __device__ __forceinline__ void topk_select_body(const TopkArgs& a, float* topk_
     const uint32_t peer = rank ^ 1u;
     const int row = blockIdx.x / C;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = max(0, min(__ldg(a.n_vis + row), a.n_cap));
+    const int n = max(0, min(ptx::ld(a.n_vis + row), a.n_cap));
     const float* g = a.scores + int64_t(row) * a.stride;
     int32_t* out = a.out + int64_t(row) * a.k;
     if (n <= a.k) {                                          // same decision in both blocks of a pair
@@ -379,7 +400,7 @@ __device__ __forceinline__ void topk_select_body(const TopkArgs& a, float* topk_
 #pragma unroll
         for (int u = 0; u < 8; ++u) {                        // eight loads in flight per thread
             const int i = i0 + u * kTopkThreads;
-            v[u] = (i < s1) ? __ldg(g + i) : CUDART_NAN_F;
+            v[u] = (i < s1) ? ptx::ld(g + i) : CUDART_NAN_F;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -489,7 +510,20 @@ __device__ __forceinline__ void topk_select_body(const TopkArgs& a, float* topk_
     if (C == 2) ptx::cluster_sync();                        // the candidate list in block 0 is complete
     if (rank != 0) return;                                  // block 0 touches no memory of block 1 from here on
     const uint32_t n_cand = sh.n_cand + peer_cand;
-    if (n_cand <= uint32_t(kTopkCand)) {
+    if (n_cand <= uint32_t(kTopkRanked)) {
+        // few candidates (the usual case: a bin is a thousandth of the range): each finds its rank by comparing itself with all the others,
+        // equal keys in the order of the list; no further barriers (the radix select takes 15)
+        if (uint32_t(tid) < n_cand) {
+            const uint32_t key = sh.cand_key[tid];
+            uint32_t rank_of = 0;
+#pragma unroll 4
+            for (uint32_t j = 0; j < n_cand; ++j) {
+                const uint32_t other = sh.cand_key[j];
+                rank_of += (other > key || (other == key && j < uint32_t(tid))) ? 1u : 0u;
+            }
+            if (rank_of < need) out[n_gt + rank_of] = sh.cand_idx[tid];
+        }
+    } else if (n_cand <= uint32_t(kTopkCand)) {
         radix_select_emit(sh, int(n_cand), need, out + n_gt, [&](int j, uint32_t& key, int32_t& idx) {
             key = sh.cand_key[j];  idx = sh.cand_idx[j];
             return true;

@@ -32,7 +32,13 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
 // its launch and set-up are hidden.  Every kernel therefore waits before it touches memory (returns at once where there
 // is nothing to wait for; after it all earlier work of the stream is complete and visible), and says early that its own
 // successor may be made resident once all of its blocks run.
+//
+// Global memory is read by plain loads (ld below), never through the read-only path (__ldg, ld.global.nc): that promises that
+// the data does not change while the kernel is resident, which the kernel before may still do, and lets the compiler move the
+// load up past the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class T>
+__device__ __forceinline__ T ld(const T* p) { return *p; }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ── mbarrier ────────────────────────────────────────────────────────────
@@ -378,9 +384,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return r;
 }
 
-__device__ __forceinline__ uint4 ldg_nc_v4(const void* p) {
+// 16 bytes that are read once
+__device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;

@@ -8,9 +8,10 @@
 // A warp takes G vectors of one row (they share the position, hence the sine and cosine); all of
 // their loads are in flight before the first is used (16-byte loads for the part that is only
 // normalised, one rotated pair per lane), and each vector is written once from registers.
-// HBM-bound when there are enough vectors; below that the time is one load latency, so the launch picks
-// the largest G in {4, 2, 1} that still gives every SM eight warps.  The frequencies come with the arguments (a double pow per
-// thread took longer than the loads): 8192 vectors of 576 from cold memory 10.4 -> 8.3 us, 64 vectors 5.9 -> 4.1 us.
+// HBM-bound when there are enough vectors; below that the time is one load latency, so the launch takes G = 2 only where
+// that still gives every SM eight warps.  The frequencies come with the arguments (a double pow per thread took longer than
+// the loads).  Cold memory: 65,536 x 16 vectors of 576 457 -> 418 us, 64 x 128 14.3 -> 10.2 us (with one vector in flight per warp);
+// G = 4 at 86 registers leaves 16 warps an SM: 483 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,7 +40,7 @@ struct RopeNormArgs {
 constexpr int kRopeNormThreads = 256;
 
 template <int G>
-__global__ void __launch_bounds__(kRopeNormThreads) rope_norm_kernel(const __grid_constant__ RopeNormArgs a) {
+__global__ void __launch_bounds__(kRopeNormThreads, 4) rope_norm_kernel(const __grid_constant__ RopeNormArgs a) {
     ptx::pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int nope = a.c - a.n_rope;
@@ -62,13 +63,13 @@ __global__ void __launch_bounds__(kRopeNormThreads) rope_norm_kernel(const __gri
         // elements [16 lane, 16 lane + 16) of the part that is not rotated, in two 16-byte halves, and the pair (lane, lane + 32) of the rest
         uint4 raw[G][2];
         __nv_bfloat16 e1[G], e2[G];
-        const int32_t position = __ldg(a.positions + row);
+        const int32_t position = ptx::ld(a.positions + row);
 #pragma unroll
         for (int j = 0; j < G; ++j) {
             if (j >= n) continue;
             const __nv_bfloat16* v = src + int64_t(j) * a.c;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) raw[j][h] = have[h] ? ptx::ldg_nc_v4(v + 16 * lane + 8 * h) : make_uint4(0, 0, 0, 0);
+            for (int h = 0; h < 2; ++h) raw[j][h] = have[h] ? ptx::ldg_stream_v4(v + 16 * lane + 8 * h) : make_uint4(0, 0, 0, 0);
             e1[j] = v[nope + lane];
             e2[j] = v[nope + kHalf + lane];
         }
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(kRopeNormThreads) rope_norm_kernel(const __gri
                 for (int h = 0; h < 2; ++h) {
                     if (!have[h]) continue;
                     float w[8];
-                    unpack8(__ldg(reinterpret_cast<const uint4*>(a.weight + 16 * lane + 8 * h)), w);
+                    unpack8(ptx::ld(reinterpret_cast<const uint4*>(a.weight + 16 * lane + 8 * h)), w);
                     float* g = f + 8 * h;
 #pragma unroll
                     for (int k = 0; k < 8; ++k) g[k] = g[k] * inv_rms * w[k];

@@ -155,3 +155,16 @@ def test_indexer_bounded_wait_runs_out_and_kernel_returns(lib):
     assert role in (0, 1, 2)
     idx, scores = run(lib, c, pages, bt, qw, c.n_vis, 256)
     check_selection(idx, scores, orc.indexer_scores(c.q_fp8, qw, pages, bt, c.n_vis), c.n_vis, 256)
+
+
+@pytest.mark.parametrize("B", [2, 80])
+@pytest.mark.parametrize("crowd", [2, 383, 384, 385, 4096, 4097])
+def test_topk_by_crowding_of_the_threshold_bin(lib, B, crowd):
+    """The threshold bin's entries are ranked by comparison up to 384, by radix select up to 4096, in place beyond: with all keys of a row
+    alike they all lie in one bin, of which half are wanted."""
+    c = orc.make_indexer_case(seed=300 + crowd, B=B, s_q=1, n=crowd)
+    c.K[:] = c.K[:, :1]
+    pages, bt, qw = indexer_inputs(c, np.random.default_rng(8))
+    idx, scores = run(lib, c, pages, bt, qw, c.n_vis, crowd // 2)
+    want = orc.indexer_scores(c.q_fp8, qw, pages, bt, c.n_vis)
+    check_selection(idx, scores, want, c.n_vis, crowd // 2)

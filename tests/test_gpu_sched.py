@@ -157,3 +157,24 @@ def test_plan_for_another_batch_is_rejected(lib):
     plan = lib.plan_csa(3, 1, 128, 256)
     with pytest.raises(ValueError):
         lib.csa_sparse_decode(plan=plan, **gu.csa_to_dev(case))
+
+
+@pytest.mark.parametrize("B,k", [(2, 512), (30, 2048), (40, 512), (60, 2048)])
+def test_plan_and_decode_back_to_back(lib, B, k):
+    """The decode kernel is launched while the planner may still run: what it reads of the plan has to be the new one.  The schedule's
+    memory holds another plan when the planner starts, and nothing comes between planner and decode; 60 rows take the merge that shares out
+    the cut units, the others the one that looks every row up."""
+    case = orc.make_csa_case(seed=400 + B, B=B, s_q=1, H=128, n_entries=k + 64, topk=k)
+    args = gu.csa_to_dev(case)
+    want, want_lse = lib.csa_sparse_decode(**args, num_splits=1)
+    lens = torch.full((B, 1), k, dtype=torch.int32, device="cuda")
+    plan = lib.plan_csa(B, 1, 128, k, topk_len=lens)
+    for _ in range(20):
+        lens.copy_(torch.randint(1, k, (B, 1), dtype=torch.int32, device="cuda"))
+        plan.remake()
+        lens.fill_(k)
+        plan.remake()
+        out, lse = lib.csa_sparse_decode(**args, plan=plan)
+    torch.cuda.synchronize()
+    assert (out.float() - want.float()).abs().max().item() <= gu.OUT_MAX_ABS
+    gu.check_lse(lse.cpu().numpy(), want_lse.cpu().numpy(), f"B={B} k={k}")
