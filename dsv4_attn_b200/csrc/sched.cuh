@@ -3,8 +3,8 @@
 //
 // A unit is (row, group of 128 heads); its work is its 64-entry tiles plus a fixed cost for the
 // set-up and the write-out of an item.  Units are laid end to end on a cost axis and the axis is cut
-// into equal parts, one per block pair (the two blocks of a pair compute the two halves of the value
-// columns of the same items).  A unit that straddles a cut is split there: each piece becomes an item
+// into equal parts, one per block pair (the two blocks of a pair own half of the
+// heads each of the same items).  A unit that straddles a cut is split there: each piece becomes an item
 // of its own with a partial-output slot, and the merge kernel adds the pieces up; a unit inside one
 // part is a single item that writes the final output directly.  With `fixed_splits` >= 1 every unit is
 // instead cut into that many equal pieces (the split count a caller asks for) and the pieces are dealt

@@ -218,7 +218,7 @@ int64_t dsv4_attn_workspace_bytes(int rows, int H, int num_splits, int64_t* lse_
  * items of 64-entry tiles so that the SMs of the device get equal shares of tiles plus per-item
  * set-up; a row that fits one share is written out directly, a row that straddles shares gets
  * partial slots that the merge adds up.  The decode entry points given that `sched` then run as
- * resident blocks (two per pair of SMs, one half of the value columns each) that walk their share
+ * resident pairs of blocks (one per two SMs, half of the heads each) that walk their share
  * of the list, keep tensor memory and barriers alive between items and fetch the next item's
  * queries and first tiles while the current one finishes.  A plan depends only on B, s_q, H and
  * the length arrays, so one plan serves every layer of a decode step that shares them.
