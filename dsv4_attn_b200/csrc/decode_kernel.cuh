@@ -1270,18 +1270,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
                 for (int i = 8; i < 32; i += 8)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) t4[j] = ptx::max3(t4[j], __uint_as_float(s0[i + 2 * j]), __uint_as_float(s0[i + 2 * j + 1]));
-                const float tmax = fmaxf(ptx::max3(t4[0], t4[1], t4[2]), t4[3]) * a.scale_log2;
+                // (of NaN logits only it is -inf: such a row moves no maximum and spoils itself alone, through its probabilities)
+                const float tmax = ptx::max3(ptx::max3(t4[0], t4[1], t4[2]), t4[3], -CUDART_INF_F) * a.scale_log2;
                 // Lazy reference maximum: move it only when the true maximum exceeds it by
                 // more than the threshold (exp2 of the excess stays <= 2^threshold).  A warp whose wait ran out comes here too
                 // and says so, so that both warps of the barrier leave the loop together.
                 float alpha = 1.f;
                 const bool moved = ptx::bar_any(pair_bar, 64, !ok || tmax > m_ref + kRescaleThreshold);
                 if (moved) {
-                    misc->exch[tid] = ok ? tmax : CUDART_NAN_F;      // (tmax is never NaN)
-                    ptx::bar_sync(pair_bar + 2u, 64);
-                    const float peer = misc->exch[tid ^ 64];
-                    if (!ok || !__all_sync(0xFFFFFFFFu, peer == peer)) { ok = false;  left = true;  break; }
-                    const float rmax = fmaxf(tmax, peer);
+                    misc->exch[tid] = tmax;
+                    // the failure travels with the barrier, apart from the data: no value of a logit can look like one
+                    if (ptx::bar_any(pair_bar + 2u, 64, !ok)) { ok = false;  left = true;  break; }
+                    const float rmax = fmaxf(tmax, misc->exch[tid ^ 64]);
                     if (rmax > m_ref + kRescaleThreshold) {       // also true for the first finite max; the same in both threads
                         alpha = (m_ref == -CUDART_INF_F) ? 0.f : ptx::ex2(m_ref - rmax);
                         m_ref = rmax;
