@@ -1211,11 +1211,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         // Thread tid owns head row tid % 64 of this block and, of its S row, the entries of block tid / 64; of its O row the value
         // columns [256 (tid / 64), +256).  The two threads of a row (same lane, warps w and w + 2) share one reference
         // maximum: they meet at a named barrier per tile, which tells whether any of its 64 threads wants to move it.
-        bool ok = wait_tmem();
-        if (!ok) report_status(a.status, kStatusWaitQ, 0, -1);
         const int r = tid & 63, colhalf = tid >> 6;
         const uint32_t lane_addr = uint32_t(warp * 32) << 16;
         const uint32_t pair_bar = 1u + uint32_t(warp & 1);
+        bool ok = wait_tmem();
+        if (!ok) report_status(a.status, kStatusWaitQ, 0, -1);
+        // (where the wait ran out for one warp of a barrier only, the other would wait for it there, without a limit)
+        ok = !ptx::bar_any(pair_bar, 64, !ok);
         // this thread's 64 bytes of a P row: 16-byte columns 4 colhalf .. +3 of row r; column c lives at (c ^ (r % 8)) << 4
         const uint32_t p_row = p_base + uint32_t(r) * 128u;
         const uint32_t p_sw = (uint32_t(4 * colhalf) ^ uint32_t(r & 7)) << 4;
