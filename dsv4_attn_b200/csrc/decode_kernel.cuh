@@ -258,6 +258,7 @@ struct SmemMisc {
     uint32_t mask[kTagRing][2];      // per tile and block: bit r = K row r takes part in the softmax
     uint32_t meta[kTagRing];
     uint32_t tmem_base;
+    uint32_t failed;                 // a wait of the pair ran out
 };
 static_assert(sizeof(SmemMisc) <= 5120, "misc area");
 
@@ -270,6 +271,22 @@ __device__ __noinline__ void report_status(int32_t* status, int code, int role, 
             status[3] = tile;
         }
     }
+}
+
+// A wait that ran out: reported, and marked (`flag`, a word of shared memory) in both blocks of the pair.
+__device__ __noinline__ void wait_ran_out(int32_t* status, uint32_t flag, int code, int role, int tile) {
+    ptx::sts_cluster_u32(ptx::mapa(flag, 0), 1u);
+    ptx::sts_cluster_u32(ptx::mapa(flag, 1), 1u);
+    report_status(status, code, role, tile);
+}
+
+// Copies and MMAs must not outlive the blocks they work for.  After an ordinary run every one has been waited for by the role that uses its result; where
+// a wait ran out that role is gone, so the block stays for a time that any copy needs less than (a few microseconds), counted from when all
+// roles have ended and none can be added.  (Waiting for their barriers instead, in the fetch and MMA warps, cost every launch 4 to 6 %.)
+constexpr uint32_t kHoldNs = 1000000u;
+__device__ __noinline__ void hold_block() {
+    const uint32_t t0 = ptx::globaltimer_lo();
+    while (ptx::globaltimer_lo() - t0 < kHoldNs) __nanosleep(1000);
 }
 
 // Development builds (-DDSV4_TRACE): block 0 records when its roles pass their pipeline points
@@ -766,6 +783,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             ptx::mbar_init(bar_id_full + 8 * i, 1);
             ptx::mbar_init(bar_id_free + 8 * i, 1);
         }
+        misc->failed = 0u;
         ptx::mbar_init(bar_tmem, 1);
         ptx::mbar_init(bar_v_free, 1);
         ptx::mbar_init(bar_q_ready, 2 * (early_q ? kNumVWarps + kNumKWarps : kNumVWarps));
@@ -800,7 +818,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     // Waits of a whole warp: the outcome is the same in all lanes (the warp-collective operations below need them all).
     auto wait_for = [&](uint32_t bar, uint32_t phase, int code, int role, int at) -> bool {
         const bool w = ptx::mbar_wait_warp(bar, phase & 1u, wait_ns);
-        if (!w) report_status(a.status, code, role, at);
+        if (!w) wait_ran_out(a.status, ptx::smem_u32(&misc->failed), code, role, at);
         return w;
     };
 
@@ -1215,7 +1233,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         const uint32_t lane_addr = uint32_t(warp * 32) << 16;
         const uint32_t pair_bar = 1u + uint32_t(warp & 1);
         bool ok = wait_tmem();
-        if (!ok) report_status(a.status, kStatusWaitQ, 0, -1);
+        if (!ok) wait_ran_out(a.status, ptx::smem_u32(&misc->failed), kStatusWaitQ, 0, -1);
         // (where the wait ran out for one warp of a barrier only, the other would wait for it there, without a limit)
         ok = !ptx::bar_any(pair_bar, 64, !ok);
         // this thread's 64 bytes of a P row: 16-byte columns 4 colhalf .. +3 of row r; column c lives at (c ^ (r % 8)) << 4
@@ -1400,6 +1418,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     ptx::cluster_sync();
     if (warp == kSWarp) {
         ptx::tc_fence_after_sync();
+        if (*reinterpret_cast<volatile uint32_t*>(&misc->failed)) hold_block();
         ptx::tmem2_dealloc(misc->tmem_base, kTmemCols);
     }
 }

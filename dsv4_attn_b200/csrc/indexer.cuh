@@ -26,7 +26,7 @@
 #include <stdint.h>
 
 #include "ptx.cuh"
-#include "decode_kernel.cuh"   // report_timeout, status codes, kDefaultWaitNs
+#include "decode_kernel.cuh"   // report_status, hold_block, status codes
 
 namespace dsv4 {
 
@@ -167,6 +167,7 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
             const bool w = i < kIdxStages || ptx::mbar_wait(bar_empty + 8 * st, uint32_t(i / kIdxStages - 1) & 1u, a.wait_ns);
             if (!__all_sync(0xFFFFFFFFu, w)) {
                 report_status(a.status, kStatusWaitIndexer, 0, tile0 + i);
+                ok = false;
                 break;
             }
             if (lane == 0) {
@@ -256,11 +257,12 @@ __global__ void __launch_bounds__(kIdxThreads, 2) indexer_logits_kernel(const __
     }
     // common exit: every role arrives; the MMA warp frees tensor memory after all accumulator reads
     ptx::tc_fence_before_sync();
-    __syncthreads();
+    const bool failed = __syncthreads_or(!ok);
     // the top-k kernel may be made resident as soon as every block of this grid is here or gone
     if (tid == 0) ptx::pdl_trigger();
     if (warp == 1) {
         ptx::tc_fence_after_sync();
+        if (failed) hold_block();                             // copies and MMAs in flight
         ptx::tmem_dealloc(tmem, kIdxTmemCols);
     }
 }

@@ -48,6 +48,59 @@ def test_bounded_wait_runs_out_and_kernel_returns(lib, with_plan):
     gu.check_lse(lse.cpu().numpy(), want_lse, "after a timed-out launch")
 
 
+@pytest.mark.parametrize("source", ["csa", "hca", "planes", "packed"])
+@pytest.mark.parametrize("tile", [0, 5, 12])
+def test_bounded_wait_at_the_start_middle_and_end_of_a_row(lib, source, tile):
+    """The first, a middle and the last tile of rows of 13 withheld: copies and MMAs are on their way, or the fetch warps have
+    already finished, when the waits run out.  The launch returns and the next one is right."""
+    n, W, H = 740, 64, 64
+    st = lib.new_status("cuda")
+    if source == "csa":
+        case = orc.make_csa_case(seed=64, B=2, s_q=1, H=H, n_entries=n + W, topk=n + W)
+        d = gu.csa_to_dev(case)
+        want = orc.csa_sparse_decode(case.q, case.pool, case.block_table, case.indices, case.sm_scale)
+        call = lambda: lib.csa_sparse_decode(status=st, num_splits=1, **d)
+    elif source == "hca":
+        case = orc.make_hca_case(seed=65, B=2, s_q=1, H=H, kv_len=n, win_len=W)
+        d = gu.hca_to_dev(case)
+        want = orc.hca_dense_decode(case.q, case.pool, case.block_table, case.kv_len, case.win, case.win_len, case.sm_scale)
+        call = lambda: lib.hca_dense_decode(status=st, num_splits=1, **d)
+    else:
+        case = orc.make_ref_layout_case(seed=66, B=2, H=H, M_cur=n, swa_len=W)
+        q, sink = gu.dev(case.Q, torch.bfloat16), gu.dev(case.sink)
+        want = orc.hca_decode_ref_layout(case.Q, case.Kc, case.Kc_s, case.Kc_rope, case.Kswa, case.Kswa_s, case.Kswa_rope, case.sink, case.sm_scale)
+        if source == "planes":
+            planes = [gu.dev(case.Kc), gu.dev(case.Kc_s), gu.dev(case.Kc_rope, torch.bfloat16), gu.dev(case.Kswa), gu.dev(case.Kswa_s),
+                      gu.dev(case.Kswa_rope, torch.bfloat16)]
+            # (no room for partials: one split)
+            call = lambda: (lib.LIB.hca_decode_fwd(*(t.data_ptr() for t in (q, *planes, sink, out)), None, None, case.sm_scale, 2, H, 448, 64, n, W,
+                                                        torch.cuda.current_stream().cuda_stream), out)[1:] + (None,)
+            out = torch.empty(2, H, 512, dtype=torch.bfloat16, device="cuda")
+        else:
+            rng = np.random.default_rng(7)
+            kv, bt = orc.pack_ref_pages(case.Kc, case.Kc_s, case.Kc_rope, 64, rng)
+            sw, sbt = orc.pack_ref_pages(case.Kswa, case.Kswa_s, case.Kswa_rope, 64, rng)
+            full = lambda v: torch.full((2,), v, dtype=torch.int32, device="cuda")
+            t = [gu.dev(kv), gu.dev(bt), full(n), gu.dev(sw), gu.dev(sbt), full(W)]
+            call = lambda: lib.hca_packed_decode(q, *t, case.sm_scale, page_size=64, attn_sink=sink, num_splits=1, status=st)
+    torch.cuda.synchronize()
+    lib.LIB.dsv4_debug_set_wait(200_000, tile)
+    try:
+        call()
+        torch.cuda.synchronize()                    # returns: no trap, no fault, no hang
+    finally:
+        lib.LIB.dsv4_debug_set_wait(0, -1)
+    if source != "planes":
+        assert st.cpu().tolist()[0] in (1, 2, 3, 4, 5, 6, 8, 9)
+    st.zero_()
+    out, lse = call()
+    torch.cuda.synchronize()
+    assert st.cpu().tolist() == [0, 0, 0, 0]
+    gu.check_out(gu.out_to_f32(out), want[0], f"{source} after a timed-out launch")
+    if lse is not None:
+        gu.check_lse(lse.cpu().numpy(), want[1], f"{source} after a timed-out launch")
+
+
 def test_csa_out_of_range_indices_and_pages_are_left_out(lib):
     case = orc.make_csa_case(seed=62, B=2, s_q=1, H=64, n_entries=[400, 400], topk=256)
     max_pages = case.block_table.shape[1]
