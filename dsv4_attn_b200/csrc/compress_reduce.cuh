@@ -96,9 +96,12 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
                 }
             }
             auto bias = [&](int j, bool bside) { return ptx::ld(reinterpret_cast<const V*>((bside ? a.B_b : a.B_a) + int64_t(j) * a.c_out + ch)); };
-            // The reference maximum is found in packed BF16 arithmetic: any value close to the true maximum serves, as long as the
-            // same one is used for every weight.  The logits themselves are formed in FP32, two channels an instruction.
+            // The reference maximum is found in packed BF16 arithmetic.  A BF16 sum is within 2^-8 of the FP32 one; raised by that much the
+            // reference is no lower than the true maximum, so that no weight exceeds 1, and while it is small (kNear) the weight of
+            // the true maximum is no smaller than 2^-1.5.  Larger logits (and infinities) take the exact maximum and differences formed
+            // before the factor log2(e): from 2^15 up the weights of finite logits would overflow or all vanish otherwise.
             constexpr int P = VEC / 2;
+            constexpr float kLog2e = 1.4426950408889634f, kNear = 128.f;
             __nv_bfloat162 pm[P];
 #pragma unroll
             for (int k = 0; k < P; ++k) pm[k] = __float2bfloat162_rn(-CUDART_INF_F);
@@ -113,44 +116,80 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
                     for (int k = 0; k < P; ++k) pm[k] = __hmax2(pm[k], __hadd2(z2[k], u2[k]));
                 }
             }
-            constexpr float kLog2e = 1.4426950408889634f;
-            const uint64_t log2e2 = ptx::pack_f32x2(kLog2e, kLog2e);
-            uint64_t nref[P], sum2[P], acc2[P];             // nref: -(reference maximum) * log2(e)
+            __nv_bfloat162 size = __habs2(pm[0]);
 #pragma unroll
-            for (int k = 0; k < P; ++k) {
-                float lo = __low2float(pm[k]), hi = __high2float(pm[k]);
-                if (!(lo > -CUDART_INF_F) || !(lo < CUDART_INF_F)) lo = 0.f;   // all -inf (or NaN): avoid inf - inf
-                if (!(hi > -CUDART_INF_F) || !(hi < CUDART_INF_F)) hi = 0.f;
-                nref[k] = ptx::pack_f32x2(-lo * kLog2e, -hi * kLog2e);
-                sum2[k] = 0ull;  acc2[k] = 0ull;
-            }
+            for (int k = 1; k < P; ++k) size = __hmax2(size, __habs2(pm[k]));
+            if (__hble2(size, __float2bfloat162_rn(kNear))) {
+                // the logits are formed in FP32, two channels an instruction
+                const uint64_t log2e2 = ptx::pack_f32x2(kLog2e, kLog2e);
+                uint64_t nref[P], sum2[P], acc2[P];         // nref: -(reference maximum) * log2(e)
 #pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                if (side == 1 && !has_b) break;
+                for (int k = 0; k < P; ++k) {
+                    const float lo = __low2float(pm[k]), hi = __high2float(pm[k]);
+                    nref[k] = ptx::pack_f32x2(fmaf(fabsf(lo), -kLog2e / 256.f, -lo * kLog2e), fmaf(fabsf(hi), -kLog2e / 256.f, -hi * kLog2e));
+                    sum2[k] = 0ull;  acc2[k] = 0ull;
+                }
 #pragma unroll
-                for (int j = 0; j < M; ++j) {
-                    float z[VEC], u[VEC], c[VEC];
-                    BfVec<VEC>::unpack(side ? zb[j] : za[j], z);
-                    BfVec<VEC>::unpack(bias(j, side == 1), u);
-                    BfVec<VEC>::unpack(side ? cb[j] : ca[j], c);
+                for (int side = 0; side < 2; ++side) {
+                    if (side == 1 && !has_b) break;
 #pragma unroll
-                    for (int k = 0; k < P; ++k) {
-                        const uint64_t t = ptx::add_f32x2(ptx::pack_f32x2(z[2 * k], z[2 * k + 1]), ptx::pack_f32x2(u[2 * k], u[2 * k + 1]));
-                        float e0, e1;
-                        ptx::unpack_f32x2(ptx::fma_f32x2(t, log2e2, nref[k]), e0, e1);
-                        const uint64_t e = ptx::pack_f32x2(ptx::ex2(e0), ptx::ex2(e1));
-                        sum2[k] = ptx::add_f32x2(sum2[k], e);
-                        acc2[k] = ptx::fma_f32x2(e, ptx::pack_f32x2(c[2 * k], c[2 * k + 1]), acc2[k]);
+                    for (int j = 0; j < M; ++j) {
+                        float z[VEC], u[VEC], c[VEC];
+                        BfVec<VEC>::unpack(side ? zb[j] : za[j], z);
+                        BfVec<VEC>::unpack(bias(j, side == 1), u);
+                        BfVec<VEC>::unpack(side ? cb[j] : ca[j], c);
+#pragma unroll
+                        for (int k = 0; k < P; ++k) {
+                            const uint64_t t = ptx::add_f32x2(ptx::pack_f32x2(z[2 * k], z[2 * k + 1]), ptx::pack_f32x2(u[2 * k], u[2 * k + 1]));
+                            float e0, e1;
+                            ptx::unpack_f32x2(ptx::fma_f32x2(t, log2e2, nref[k]), e0, e1);
+                            const uint64_t e = ptx::pack_f32x2(ptx::ex2(e0), ptx::ex2(e1));
+                            sum2[k] = ptx::add_f32x2(sum2[k], e);
+                            acc2[k] = ptx::fma_f32x2(e, ptx::pack_f32x2(c[2 * k], c[2 * k + 1]), acc2[k]);
+                        }
                     }
                 }
-            }
 #pragma unroll
-            for (int k = 0; k < P; ++k) {
-                float s0, s1, a0, a1;
-                ptx::unpack_f32x2(sum2[k], s0, s1);
-                ptx::unpack_f32x2(acc2[k], a0, a1);
-                o[2 * k] = a0 / s0;
-                o[2 * k + 1] = a1 / s1;
+                for (int k = 0; k < P; ++k) {
+                    float s0, s1, a0, a1;
+                    ptx::unpack_f32x2(sum2[k], s0, s1);
+                    ptx::unpack_f32x2(acc2[k], a0, a1);
+                    o[2 * k] = a0 / s0;
+                    o[2 * k + 1] = a1 / s1;
+                }
+            } else {
+                float zmax[VEC], sum[VEC], acc[VEC];
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) { zmax[k] = -CUDART_INF_F;  sum[k] = 0.f;  acc[k] = 0.f; }
+#pragma unroll
+                for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+                    for (int side = 0; side < 2; ++side) {
+                        if (side == 1 && !has_b) break;
+#pragma unroll
+                        for (int j = 0; j < M; ++j) {
+                            float z[VEC], u[VEC], c[VEC];
+                            BfVec<VEC>::unpack(side ? zb[j] : za[j], z);
+                            BfVec<VEC>::unpack(bias(j, side == 1), u);
+                            BfVec<VEC>::unpack(side ? cb[j] : ca[j], c);
+#pragma unroll
+                            for (int k = 0; k < VEC; ++k) {
+                                if (pass == 0) {
+                                    zmax[k] = fmaxf(zmax[k], z[k] + u[k]);
+                                } else {
+                                    const float e = ptx::ex2((z[k] + u[k] - zmax[k]) * kLog2e);
+                                    sum[k] += e;
+                                    acc[k] = fmaf(e, c[k], acc[k]);
+                                }
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k)
+                        if (pass == 0 && !(fabsf(zmax[k]) < CUDART_INF_F)) zmax[k] = 0.f;      // all -inf (or NaN): avoid inf - inf
+                }
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) o[k] = acc[k] / sum[k];
             }
         } else {
             float z[2 * M], c[2 * M];

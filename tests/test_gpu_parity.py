@@ -287,6 +287,48 @@ def test_compress_reduce_vs_reference_kernel_and_errors(lib):
         lib.csa_compress_reduce_fwd(*[x[:, :4095].contiguous() if x.dim() == 3 else x for x in t], 4)
 
 
+LOGIT_SIZES = [1.0, 60.0, 300.0, 2.0 ** 14, 2.0 ** 15, 2.0 ** 20, 1e30, 1e38]
+
+
+def wide_logits(rng, shape, size):
+    """Gating logits of the given size; rows masked with -inf and, one block of 16 rows, with the type's lowest value."""
+    z = orc.bf16_round((rng.standard_normal(shape) * size).clip(-3e38, 3e38).astype(np.float32))
+    z[:, 4:8, ::3] = -np.inf                                   # masked rows, in some channels
+    z[:, 16:32, 1::4] = np.float32(-3.3895314e38)
+    z[:, 9, 5] = np.inf                                        # NaN out, as in the reference's softmax
+    return z
+
+
+def check_compressed(got_bits, want_bits, biggest):
+    """A BF16 place apart (2^-7 at most), and 2^-17 of the largest value that was weighted: a weight above 2^-24 of the sum has an exponent
+    below 24 in size, rounded to 2^-20 in FP32; 2^-3 for the exponential itself and the order of the sums."""
+    got, want = gu.bits_to_f32(got_bits), gu.bits_to_f32(want_bits)
+    assert np.array_equal(np.isnan(got), np.isnan(want)), "NaN pattern differs"
+    fin = ~np.isnan(want)
+    err = np.abs(got[fin].astype(np.float64) - want[fin])
+    assert (err <= 2.0 ** -7 * np.abs(want[fin]).astype(np.float64) + 2.0 ** -17 * float(biggest)).all(), err.max()
+
+
+@pytest.mark.parametrize("c_out", [64, 33])
+@pytest.mark.parametrize("size", LOGIT_SIZES)
+def test_compress_reduce_with_large_and_masked_logits(lib, size, c_out):
+    """The softmax over the gating logits holds for every finite logit, next to channels with small ones in the same thread."""
+    rng = np.random.default_rng(62)
+    B, n = 2, 64
+    c = orc.make_compress_case(seed=63, B=B, n=n, c_out=c_out)
+    Z = []
+    for _ in range(2):
+        z = wide_logits(rng, (B, n, c_out), size)
+        z[..., 2::8] = orc.bf16_round(rng.standard_normal((B, n, len(range(2, c_out, 8)))).astype(np.float32))
+        Z.append(z)
+    C = [x * np.float32(2.0 ** 118 if size >= 2 ** 14 else 1.0) for x in (c.C_a, c.C_b)]
+    bf = lambda a: gu.dev(a, torch.bfloat16)
+    out = lib.csa_compress_reduce_fwd(*[bf(x) for x in (*C, *Z, c.B_a, c.B_b)], 4)
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = orc.compress_reduce(*C, *Z, c.B_a, c.B_b, 4)
+    check_compressed(out.view(torch.int16).cpu().numpy().view(np.uint16), want, max(np.abs(x).max() for x in C))
+
+
 def test_more_than_128_heads_and_partial_head_group(lib):
     """H = 192: two groups of 128 head rows, the second only half used."""
     case = orc.make_csa_case(seed=71, B=2, s_q=1, H=192, n_entries=300, topk=256)
