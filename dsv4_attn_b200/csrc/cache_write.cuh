@@ -119,14 +119,10 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
     const int rows_per = (a.m + kHcaRowGroups - 1) / kHcaRowGroups;
     const int r0 = rg * rows_per, r1 = min(r0 + rows_per, a.m);
 
-    // The running maximum starts at a large negative finite value instead of -inf, so that the
-    // update below needs no special cases: with it every difference stays finite, a logit of -inf
-    // gets weight zero, and a block whose logits are all -inf ends with a zero denominator (NaN
-    // out, as in the reference's softmax).
-    constexpr float kLowest = -1e30f;
+    // A block whose logits are all -inf, or hold +inf, gives NaN, as in the reference's softmax.
     float mx[8], l[8], acc[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { mx[k] = kLowest;  l[k] = 0.f;  acc[k] = 0.f; }
+    for (int k = 0; k < 8; ++k) { mx[k] = -CUDART_INF_F;  l[k] = 0.f;  acc[k] = 0.f; }
     if (active) {
         const int64_t base = int64_t(b) * a.stride_b + int64_t(blk) * a.m * a.stride_n + ch;
         // one step = kHcaBatch rows; FULL: all of them exist (no per-row predicates in the code)
@@ -142,12 +138,15 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
                 }
             }
             // The reference maximum of the step is found in packed BF16 arithmetic (one add and
-            // one max per two elements): any value close to the true maximum serves, as long as
+            // one max per two elements): a value close to the true maximum serves, as long as
             // the same one is used for every weight of the step.  Only the raw vectors stay in
-            // registers; the logits themselves are formed in FP32 below.
+            // registers; the logits themselves are formed in FP32 below.  A BF16 sum is within 2^-8 of the FP32 one: up to kNear no weight
+            // exceeds 2^0.75 and the largest is no smaller than 2^-0.75.  Larger logits (and infinities) take the exact maximum and
+            // differences formed before the factor log2(e): from 2^15 up the weights of finite logits would overflow or all vanish otherwise.
+            constexpr float kNear = 128.f;
             __nv_bfloat162 pm[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) pm[k] = __float2bfloat162_rn(kLowest);
+            for (int k = 0; k < 4; ++k) pm[k] = __float2bfloat162_rn(-CUDART_INF_F);
 #pragma unroll
             for (int j = 0; j < kHcaBatch; ++j) {
                 if (FULL || r + j < r1) {
@@ -156,6 +155,42 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
 #pragma unroll
                     for (int k = 0; k < 4; ++k) pm[k] = __hmax2(pm[k], __hadd2(z2[k], u2[k]));
                 }
+            }
+            if (!__hble2(__hmax2(__hmax2(__habs2(pm[0]), __habs2(pm[1])), __hmax2(__habs2(pm[2]), __habs2(pm[3]))), __float2bfloat162_rn(kNear))) {
+                float ref[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) ref[k] = mx[k];
+#pragma unroll
+                for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+                    for (int j = 0; j < kHcaBatch; ++j) {
+                        if (FULL || r + j < r1) {
+                            float z[8], u[8], cf[8];
+                            unpack8(zv[j], z);
+                            unpack8(bv[j], u);
+                            unpack8(cv[j], cf);
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                if (pass == 0) {
+                                    ref[k] = fmaxf(ref[k], z[k] + u[k]);
+                                } else {
+                                    const float e = ptx::ex2((z[k] + u[k] - ref[k]) * kLog2e);
+                                    l[k] += e;
+                                    acc[k] = fmaf(e, cf[k], acc[k]);
+                                }
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        if (pass == 1) break;
+                        const float top = ref[k];
+                        if (!(fabsf(top) < CUDART_INF_F)) ref[k] = 0.f;              // all -inf so far, or +inf: avoid inf - inf
+                        const float w = ptx::ex2((mx[k] - ref[k]) * kLog2e);
+                        l[k] *= w;  acc[k] *= w;  mx[k] = top;
+                    }
+                }
+                return;
             }
             float nref[8];                       // -(new reference maximum) * log2(e)
 #pragma unroll

@@ -12,6 +12,7 @@ pytestmark = pytest.mark.gpu
 
 from oracle import dsv4_oracle as orc  # noqa: E402
 from tests import gpu_util as gu  # noqa: E402
+from tests.test_gpu_parity import LOGIT_SIZES, check_compressed, wide_logits  # noqa: E402
 
 GOLD = Path(__file__).resolve().parent / "golden"
 
@@ -52,6 +53,25 @@ def test_hca_compress_vs_reference_outputs(lib, name):
     assert got.shape == z["out"].shape
     assert bf16_ulp_diff(got, orc.f32_to_bf16_bits(z["out"])).max() <= 1
     assert bf16_ulp_diff(got, orc.f32_to_bf16_bits(orc.hca_compress(c.C, c.Z, c.bias, c.m))).max() <= 1
+
+
+@pytest.mark.parametrize("m", [128, 7])
+@pytest.mark.parametrize("size", LOGIT_SIZES)
+def test_hca_compress_with_large_and_masked_logits(lib, size, m):
+    """The softmax over the gating logits holds for every finite logit, next to channels with small ones in the same thread."""
+    rng = np.random.default_rng(64)
+    B, n = 2, 2 * m if m > 100 else 12 * m
+    c = orc.make_hca_compress_case(seed=65, B=B, n=n, c=64, m=m)
+    Z = wide_logits(rng, (B, n, 64), size)
+    Z[..., 2::8] = orc.bf16_round(rng.standard_normal((B, n, 8)).astype(np.float32))
+    if m > 100:
+        Z[1, :m, 1::4] = np.float32(-3.3895314e38)            # a block masked with the type's lowest value
+        Z[0, m:, 6] = -np.inf                                 # a block masked with -inf: NaN
+    out = lib.hca_compress_fwd(bf(c.C), bf(Z), bf(c.bias), m)
+    torch.cuda.synchronize()
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = orc.hca_compress(c.C, Z, c.bias, m)
+    check_compressed(out.view(torch.int16).cpu().numpy().view(np.uint16), orc.f32_to_bf16_bits(want), np.abs(c.C).max())
 
 
 def test_kv_quantize_insert_bit_exact(lib):
