@@ -192,12 +192,12 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_sched_kernel(const
     __shared__ int s_unit[kChunk];
     __shared__ int s_count[kCombineWarps];
     ptx::pdl_trigger();
+    ptx::pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_units = a.N * a.hgs;
     const int slices = (min(a.H, 128) + kCombineWarps - 1) / kCombineWarps;
     int64_t job0 = 0;                         // jobs (cut unit, eight heads) of the chunks before this one
     for (int base = 0; base < n_units; base += kChunk) {
-        // The plan is read ahead of the wait below: the decode kernel, whose blocks have all started by now, waited for it.
         uint32_t cut[kPerThread];             // which units of the warp's 128 are cut
         int mine = 0;
 #pragma unroll
@@ -222,7 +222,6 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_sched_kernel(const
         }
         __syncthreads();
         const int jobs = count * slices;
-        if (base == 0) ptx::pdl_wait();
         int64_t first = (int64_t(blockIdx.x) - job0) % int64_t(gridDim.x);
         if (first < 0) first += gridDim.x;
         for (int64_t j = first; j < jobs; j += gridDim.x) {
