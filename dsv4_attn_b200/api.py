@@ -100,13 +100,15 @@ class Plan:
         self.partial_o = torch.empty(max(po.value // 4, 4), dtype=torch.float32, device=device)
         self.partial_lse = torch.empty(max(pl.value // 4, 4), dtype=torch.float32, device=device)
         self.lengths = lengths
-        # what the decode calls and remake() take of a plan
-        self.fast = (kind, B, s_q, H, topk, self.sched, self.partial_o, self.partial_lse)
-        self._request = (kind, B, s_q, H, topk, num_splits, num_sms, *lengths, self.sched)
         self.remake()
 
+    @property
+    def fast(self):
+        """What the decode calls take of a plan (read anew for each: the attributes are the caller's to change)."""
+        return (self.kind, self.B, self.s_q, self.H, self.topk, self.sched, self.partial_o, self.partial_lse)
+
     def remake(self):
-        rc = _host.plan(*self._request)
+        rc = _host.plan(self.kind, self.B, self.s_q, self.H, self.topk, self.num_splits, self.num_sms, *self.lengths, self.sched)
         if rc == 0:
             return self
         topk_len, kv_len, win_len = self.lengths

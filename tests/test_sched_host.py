@@ -146,3 +146,27 @@ def test_rejected_requests():
     assert b"smaller" in _lib.LIB.dsv4_attn_last_error()
     p = _lib.PlanParams(kind=7, B=4, s_q=1, H=128, topk=512, num_splits=0, num_sms=148, sched=buf.ctypes.data, sched_bytes=1 << 20)
     assert _lib.LIB.dsv4_attn_plan_host(C.byref(p)) == 1
+
+
+def test_plan_object_follows_its_attributes(monkeypatch):
+    """remake() and the decode calls take what the plan holds when they run, not what it held when it was made."""
+    import torch
+    from dsv4_attn_b200 import api
+    calls = []
+
+    class Host:
+        @staticmethod
+        def plan(*args):
+            calls.append(args)
+            return 0
+
+    monkeypatch.setattr(api, "_host", Host)
+    kv = torch.zeros(4, 1, dtype=torch.int32)
+    plan = api.Plan(0, 4, 1, 128, 512, 0, 148, (None, kv, None), "cpu")
+    assert calls[-1][7:] == (None, kv, None, plan.sched)
+    other, sched, po = kv + 1, plan.sched.clone(), plan.partial_o.clone()
+    plan.lengths = (None, other, None)
+    plan.sched, plan.partial_o = sched, po
+    plan.remake()
+    assert calls[-1][8] is other and calls[-1][10] is sched
+    assert plan.fast[5] is sched and plan.fast[6] is po and plan.fast[7] is plan.partial_lse
