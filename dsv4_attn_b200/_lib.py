@@ -183,4 +183,20 @@ def _load() -> C.CDLL:
     return lib
 
 
+def load_host():
+    """The native half of the operator surface (csrc/host.cpp), for this Python and this torch."""
+    import importlib.machinery
+    import importlib.util
+
+    from .build import host_path
+    path = host_path()
+    if not path.exists():
+        raise LibraryNotBuilt(f"{path.name} not found (the native module is built per Python and torch version); build it with `python -m dsv4_attn_b200.build`")
+    name = f"{__package__}._host"
+    spec = importlib.util.spec_from_file_location(name, path, loader=importlib.machinery.ExtensionFileLoader(name, str(path)))
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 LIB = _load()

@@ -18,10 +18,11 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _host, _lib
+from . import _lib
 from .layout import D_QK, D_LATENT, ENTRY_BYTES, PAGE_ENTRIES
 
 MAX_SPLITS = 64
+_host = _lib.load_host()
 
 
 class Dsv4Error(RuntimeError):

@@ -1,6 +1,7 @@
 #!/usr/bin/env python3
 """Build the two shared objects in-tree: libdsv4_attn.so (the kernels behind their C ABI; plain nvcc, no torch) and
-_host.so (the Python operator surface's fast path; g++ against torch's headers).
+_host.<python>.torch-<version>.so (the Python operator surface's fast path; g++ against torch's headers, hence one
+file per version of both).
 
     python -m dsv4_attn_b200.build            # builds what is out of date
     python -m dsv4_attn_b200.build --ptxas-v  # also prints registers / spills / shared memory
@@ -23,7 +24,6 @@ SOURCE = HERE / "csrc" / "api.cu"
 OUT = HERE / "libdsv4_attn.so"
 HEADER = HERE.parent / "include" / "dsv4_attn.h"
 HOST_SOURCE = HERE / "csrc" / "host.cpp"
-HOST_OUT = HERE / "_host.so"
 DEPS = [p for p in sorted((HERE / "csrc").glob("*")) if p != HOST_SOURCE] + [HEADER]
 
 
@@ -34,9 +34,16 @@ def needs_build(out: Path = OUT, deps=tuple(DEPS)) -> bool:
     return any(p.stat().st_mtime > t for p in deps)
 
 
+def host_path() -> Path:
+    """The native module's file: it is compiled against torch's C++ classes and Python's ABI, so it serves the versions it was built for only."""
+    import torch
+    return HERE / f"_host.{sys.implementation.cache_tag}.torch-{torch.__version__}.so"
+
+
 def build_host(force: bool = False, quiet: bool = False) -> Path:
-    if not force and not needs_build(HOST_OUT, (HOST_SOURCE, HEADER)):
-        return HOST_OUT
+    out = host_path()
+    if not force and not needs_build(out, (HOST_SOURCE, HEADER)):
+        return out
     import sysconfig
 
     import torch
@@ -45,12 +52,12 @@ def build_host(force: bool = False, quiet: bool = False) -> Path:
     cuda = Path(nvcc).resolve().parent.parent
     cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            f"-I{sysconfig.get_paths()['include']}", "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
-           "-isystem", str(cuda / "include"), "-o", str(HOST_OUT), str(HOST_SOURCE), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+           "-isystem", str(cuda / "include"), "-o", str(out), str(HOST_SOURCE), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
            "-ltorch", "-ltorch_python"]
     if not quiet:
         print(" ".join(cmd), flush=True)
     subprocess.run(cmd, check=True)
-    return HOST_OUT
+    return out
 
 
 def build(force: bool = False, ptxas_v: bool = False, quiet: bool = False) -> Path:

@@ -84,3 +84,18 @@ def test_planner_is_host_only_and_sane():
     n = _lib.LIB.dsv4_attn_workspace_bytes(256, 128, 8, ctypes.byref(off))
     assert off.value == 8 * 256 * 128 * 512 * 4 and n >= off.value + 8 * 256 * 128 * 4
     assert _lib.LIB.dsv4_attn_workspace_bytes(256, 128, 1, None) == 0
+
+
+def test_native_module_is_built_and_loaded_per_python_and_torch(monkeypatch):
+    """It is compiled against torch's C++ classes: the file of another torch or Python is neither taken for up to date nor loaded."""
+    import sys
+
+    import torch
+    from dsv4_attn_b200 import _lib, build
+    path = build.build_host(quiet=True)
+    assert sys.implementation.cache_tag in path.name and torch.__version__ in path.name
+    assert not build.needs_build(path, (build.HOST_SOURCE, build.HEADER)) and hasattr(_lib.load_host(), "bind")
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.host_path() != path and build.needs_build(build.host_path(), (build.HOST_SOURCE, build.HEADER))
+    with pytest.raises(_lib.LibraryNotBuilt):
+        _lib.load_host()
