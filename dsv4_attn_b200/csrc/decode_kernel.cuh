@@ -258,9 +258,8 @@ struct SmemMisc {
     uint32_t mask[kTagRing][2];      // per tile and block: bit r = K row r takes part in the softmax
     uint32_t meta[kTagRing];
     uint32_t tmem_base;
-    uint32_t failed;                 // a wait of the pair ran out
 };
-static_assert(sizeof(SmemMisc) <= 5120, "misc area");
+static_assert(sizeof(SmemMisc) <= 5120 - 16, "misc area; the last word of the block's shared memory is failed_flag()");
 
 // (out of line: it is called from many places and hardly ever runs)
 __device__ __noinline__ void report_status(int32_t* status, int code, int role, int tile) {
@@ -273,10 +272,19 @@ __device__ __noinline__ void report_status(int32_t* status, int code, int role, 
     }
 }
 
-// A wait that ran out: reported, and marked (`flag`, a word of shared memory) in both blocks of the pair.
-__device__ __noinline__ void wait_ran_out(int32_t* status, uint32_t flag, int code, int role, int tile) {
-    ptx::sts_cluster_u32(ptx::mapa(flag, 0), 1u);
-    ptx::sts_cluster_u32(ptx::mapa(flag, 1), 1u);
+// Set when a wait of the pair has run out: the last word of a block's dynamic shared memory (found without an argument, which would
+// take a register at every wait: HCA, 64 requests, 32.0 us instead of 32.3).
+__device__ __forceinline__ uint32_t failed_flag() {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint32_t bytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+    return ptx::smem_u32(smem_raw) + bytes - 4u;
+}
+
+// A wait that ran out: reported, and marked in both blocks of the pair.
+__device__ __noinline__ void wait_ran_out(int32_t* status, int code, int role, int tile) {
+    ptx::sts_cluster_u32(ptx::mapa(failed_flag(), 0), 1u);
+    ptx::sts_cluster_u32(ptx::mapa(failed_flag(), 1), 1u);
     report_status(status, code, role, tile);
 }
 
@@ -783,7 +791,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             ptx::mbar_init(bar_id_full + 8 * i, 1);
             ptx::mbar_init(bar_id_free + 8 * i, 1);
         }
-        misc->failed = 0u;
+        ptx::sts_u32(failed_flag(), 0u);
         ptx::mbar_init(bar_tmem, 1);
         ptx::mbar_init(bar_v_free, 1);
         ptx::mbar_init(bar_q_ready, 2 * (early_q ? kNumVWarps + kNumKWarps : kNumVWarps));
@@ -818,7 +826,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     // Waits of a whole warp: the outcome is the same in all lanes (the warp-collective operations below need them all).
     auto wait_for = [&](uint32_t bar, uint32_t phase, int code, int role, int at) -> bool {
         const bool w = ptx::mbar_wait_warp(bar, phase & 1u, wait_ns);
-        if (!w) wait_ran_out(a.status, ptx::smem_u32(&misc->failed), code, role, at);
+        if (!w) wait_ran_out(a.status, code, role, at);
         return w;
     };
 
@@ -1233,7 +1241,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         const uint32_t lane_addr = uint32_t(warp * 32) << 16;
         const uint32_t pair_bar = 1u + uint32_t(warp & 1);
         bool ok = wait_tmem();
-        if (!ok) wait_ran_out(a.status, ptx::smem_u32(&misc->failed), kStatusWaitQ, 0, -1);
+        if (!ok) wait_ran_out(a.status, kStatusWaitQ, 0, -1);
         // (where the wait ran out for one warp of a barrier only, the other would wait for it there, without a limit)
         ok = !ptx::bar_any(pair_bar, 64, !ok);
         // this thread's 64 bytes of a P row: 16-byte columns 4 colhalf .. +3 of row r; column c lives at (c ^ (r % 8)) << 4
@@ -1418,7 +1426,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
     ptx::cluster_sync();
     if (warp == kSWarp) {
         ptx::tc_fence_after_sync();
-        if (*reinterpret_cast<volatile uint32_t*>(&misc->failed)) hold_block();
+        if (ptx::lds_u32(failed_flag())) hold_block();
         ptx::tmem2_dealloc(misc->tmem_base, kTmemCols);
     }
 }
