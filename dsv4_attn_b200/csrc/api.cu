@@ -1,8 +1,8 @@
 // C ABI of the library: argument validation, parameter filling, launches.
 // No allocation and no synchronisation.  Process-wide state is limited to: per-device flags that a
-// kernel's shared-memory attribute has been set, the per-device address of the built-in scratch array of
-// the entry point that allocates nothing (both written once, atomically), and the test switches of
-// dsv4_debug_set_flags / dsv4_debug_set_wait, which are read once per call.
+// kernel's shared-memory attribute has been set, per-device SM counts, the per-device address of the built-in scratch array of
+// the entry point that allocates nothing (all written once, atomically), each thread's RoPE frequencies of the theta it used
+// last, and the test switches of dsv4_debug_set_flags / dsv4_debug_set_wait, which are read once per call.
 #include "../../include/dsv4_attn.h"
 
 #include <cuda.h>
@@ -93,35 +93,15 @@ cudaError_t make_page_map(CUtensorMap* map, const void* base, int64_t pages, int
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// The record maps of one pool (DecodeArgs::rec_map, rope_map).  A map is a function of the pool's address, rows and kind alone, and a
-// program's pools stay where they are from call to call, so each thread keeps the last few it made (2 us a call otherwise).
-struct PoolMaps {
-    const void* lat = nullptr;
-    const void* rope = nullptr;
-    int64_t rows = 0;
-    int src = -1, page = 0;
-    CUtensorMap rec[3], rope_map;
-};
+// The record maps of one pool (DecodeArgs::rec_map, rope_map), made for the call: nothing is kept by an address.
 // (page: tokens per page where the rows are pages)
-cudaError_t pool_maps(const PoolMaps** out, const void* lat, const void* rope, int64_t rows, int src, int page) {
-    constexpr int kKept = 8;
-    static thread_local PoolMaps kept[kKept];
-    static thread_local int next = 0;
-    for (const PoolMaps& m : kept)
-        if (m.lat == lat && m.rope == rope && m.rows == rows && m.src == src && m.page == page) { *out = &m;  return cudaSuccess; }
+cudaError_t pool_maps(CUtensorMap (&rec)[3], CUtensorMap& rope_map, const void* lat, const void* rope, int64_t rows, bool ref, int page) {
     if (rows > 0x7FFFFFFF) return cudaErrorInvalidValue;                   // TMA coordinates are 32-bit
-    PoolMaps& m = kept[next];
-    m.lat = nullptr;
-    const bool ref = src == kSrcRef;
     const int pitch = page ? 576 : (ref ? 448 : 656), boxes[3] = {pitch, 256, page ? 320 : (ref ? 192 : 16)};
     cudaError_t e = cudaSuccess;
     for (int j = 0; j < 3 && e == cudaSuccess; ++j)
-        e = page ? make_page_map(&m.rec[j], lat, rows, page, boxes[j]) : make_row_map(&m.rec[j], lat, rows, pitch, boxes[j]);
-    if (e == cudaSuccess && ref) e = make_row_map(&m.rope_map, rope, rows, 128, 128);
-    if (e != cudaSuccess) return e;
-    m.lat = lat;  m.rope = rope;  m.rows = rows;  m.src = src;  m.page = page;
-    next = (next + 1) % kKept;
-    *out = &m;
+        e = page ? make_page_map(&rec[j], lat, rows, page, boxes[j]) : make_row_map(&rec[j], lat, rows, pitch, boxes[j]);
+    if (e == cudaSuccess && ref) e = make_row_map(&rope_map, rope, rows, 128, 128);
     return e;
 }
 
@@ -129,18 +109,13 @@ cudaError_t pool_maps(const PoolMaps** out, const void* lat, const void* rope, i
 template <int SRC>
 cudaError_t make_record_maps(DecodeArgs& a) {
     constexpr bool ref = SRC == kSrcRef, paged = SRC == kSrcRefPaged;
-    // (the CSA and HCA sources read the same records: one set of maps for a pool)
-    constexpr int kind = is_ref_layout(SRC) ? SRC : int(kSrcCsa);
     const struct { const void* lat;  const void* rope;  int64_t rows; } pools[2] = {
         {paged ? a.pg_kv : (ref ? a.ref_kc : a.kv_pool), a.ref_kc_rope, paged ? a.pg_num_pages : (ref ? int64_t(a.B) * a.ref_m_cur : int64_t(a.num_pages) * 64)},
         {paged ? a.pg_swa : (ref ? a.ref_ks : a.win_pool), a.ref_ks_rope, paged ? a.pg_swa_num_pages : (ref ? int64_t(a.B) * a.ref_swa_len : int64_t(a.B) * a.win_cap)}};
     for (int i = 0; i < 2; ++i) {
         if (pools[i].lat == nullptr || pools[i].rows <= 0) continue;
-        const PoolMaps* m = nullptr;
-        const cudaError_t e = pool_maps(&m, pools[i].lat, pools[i].rope, pools[i].rows, kind, paged ? 1 << a.pg_page_shift : 0);
+        const cudaError_t e = pool_maps(a.rec_map[i], a.rope_map[i], pools[i].lat, pools[i].rope, pools[i].rows, ref, paged ? 1 << a.pg_page_shift : 0);
         if (e != cudaSuccess) return e;
-        for (int j = 0; j < 3; ++j) a.rec_map[i][j] = m->rec[j];
-        if (ref) a.rope_map[i] = m->rope_map;
     }
     return cudaSuccess;
 }

@@ -48,3 +48,19 @@ def test_nothing_is_read_before_the_wait_on_the_previous_kernel(name):
     assert wait is not None, "no unconditional wait"
     early = re.search(r"ptx::(ld|ldg|tma_load|tma_gather|bulk_load)\w*\(|plan_row_lengths\(", body[:wait.start()])
     assert early is None, f"{name} reads before its wait: {body[early.start():early.start() + 60]}"
+
+
+# What may outlive a call: facts about the device or the process, and the frequencies of the theta last used.
+KEPT = {"fn", "known", "done", "done_topk", "done_pair", "per_device", "dummy", "known_theta", "known_freq"}
+SWITCHES = {"g_dbg", "g_wait_ns", "g_drop_tile", "g_trace", "t_last_error"}
+
+
+def test_nothing_is_kept_by_an_address_between_calls():
+    """State of the host side is what the list says: no tensor map, workspace or check is remembered for a buffer seen before."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "api.cu").read_text())
+    inside = set()
+    for m in re.finditer(r"\bstatic (?!constexpr)(?:thread_local )?(?:std::atomic<[^>]+>|\w+) ([^;({]+)(?=[;{])", text):
+        inside |= {re.match(r"\w+", part.strip()).group(0) for part in m.group(1).split(",")}
+    assert inside == KEPT, inside ^ KEPT
+    outside = set(re.findall(r"^(?:std::atomic<[^\n]+>|thread_local [^\n=]*?) ?(\w+)(?:\{| =)", text, flags=re.M))
+    assert outside == SWITCHES, outside ^ SWITCHES
