@@ -56,10 +56,12 @@ def _rc(rc: int, what: str) -> None:
         raise Dsv4Error(f"{what} failed: cudaError={rc}")
 
 
-_host.bind(*(C.cast(getattr(_lib.LIB, name), C.c_void_p).value for name in (
+# in the order of struct Library in csrc/host.cpp
+ENTRY_POINTS = (
     "dsv4_csa_sparse_decode_fwd", "dsv4_hca_dense_decode_fwd", "dsv4_hca_packed_decode_fwd", "hca_decode_fwd", "dsv4_rope_norm_fwd",
     "dsv4_kv_quantize_insert", "dsv4_csa_compress_reduce_fwd", "dsv4_hca_compress_fwd", "dsv4_indexer_topk_fwd", "dsv4_attn_combine",
-    "dsv4_attn_plan", "dsv4_attn_plan_splits")))
+    "dsv4_attn_plan", "dsv4_attn_plan_splits")
+_host.bind(*(C.cast(getattr(_lib.LIB, name), C.c_void_p).value for name in ENTRY_POINTS))
 
 
 def plan_splits(rows: int, H: int, max_len: int, num_sms: int = 0) -> int:

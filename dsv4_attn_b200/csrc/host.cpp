@@ -69,7 +69,20 @@ bool number(PyObject* o, float* v) {
 }
 bool fits32(int64_t v) { return v >= 0 && v <= 0x7FFFFFFF; }
 void* stream_of(const at::Tensor* t) { return c10::cuda::getCurrentCUDAStream(t->device().index()).stream(); }
-at::Tensor empty(at::IntArrayRef s, at::ScalarType type, const at::Tensor* like) { return at::Tensor(at::detail::empty_cuda(s, type, like->device(), std::nullopt)); }
+// Other Python threads run while the allocator or a launch makes this one wait (the launch queue may be full of work that one of them has to feed).
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+template <typename... P, typename... A>
+int launch(int (*entry)(P...), A&&... args) {
+    NoGil released;
+    return entry(args...);
+}
+at::Tensor empty(at::IntArrayRef s, at::ScalarType type, const at::Tensor* like) {
+    NoGil released;
+    return at::Tensor(at::detail::empty_cuda(s, type, like->device(), std::nullopt));
+}
 
 // An output the caller passed (checked) or that is allocated here; result() hands it to Python.
 struct Output {
@@ -176,7 +189,7 @@ PyObject* csa(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.kv_len = ptr<int32_t>(kv_len);  p.topk_len = ptr<int32_t>(topk_len);  p.attn_sink = ptr<float>(d.sink);
     p.out = ptr(d.out.t);  p.lse = ptr<float>(d.lse.t);  p.partial_o = ptr<float>(d.po);  p.partial_lse = ptr<float>(d.pl);
     p.status = ptr<int32_t>(d.status);  p.sched = d.sched;
-    const int rc = lib.csa(&p, stream_of(d.q));
+    const int rc = launch(lib.csa, &p, stream_of(d.q));
     return rc != 0 ? code(rc) : pair(d.out, d.lse);
 }
 
@@ -199,7 +212,7 @@ PyObject* hca(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.win_pool = ptr(win);  p.win_len = ptr<int32_t>(win_len);  p.attn_sink = ptr<float>(d.sink);
     p.out = ptr(d.out.t);  p.lse = ptr<float>(d.lse.t);  p.partial_o = ptr<float>(d.po);  p.partial_lse = ptr<float>(d.pl);
     p.status = ptr<int32_t>(d.status);  p.sched = d.sched;
-    const int rc = lib.hca(&p, stream_of(d.q));
+    const int rc = launch(lib.hca, &p, stream_of(d.q));
     return rc != 0 ? code(rc) : pair(d.out, d.lse);
 }
 
@@ -245,7 +258,7 @@ PyObject* packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.q = ptr(q);  p.kv_pages = ptr(pool[0]);  p.block_table = ptr<int32_t>(table[0]);  p.m_cur = ptr<int32_t>(m_cur);
     p.swa_pages = ptr(pool[1]);  p.swa_block_table = ptr<int32_t>(table[1]);  p.swa_len = ptr<int32_t>(swa_len);
     p.attn_sink = ptr<float>(sink);  p.out = ptr(out.t);  p.lse = ptr<float>(lse.t);  p.status = ptr<int32_t>(status);
-    const int rc = lib.packed(&p, stream_of(q));
+    const int rc = launch(lib.packed, &p, stream_of(q));
     return rc != 0 ? code(rc) : pair(out, lse);
 }
 
@@ -279,7 +292,7 @@ PyObject* planes(PyObject*, PyObject* const* a, Py_ssize_t n) {
         po = &own_po;
         pl = &own_pl;
     }
-    const int rc = lib.planes(ptr(q), ptr(t[0]), ptr(t[1]), ptr(t[2]), ptr(t[3]), ptr(t[4]), ptr(t[5]), ptr(t[6]), ptr(o), ptr(po), ptr(pl), sm_scale, int(B), int(H),
+    const int rc = launch(lib.planes, ptr(q), ptr(t[0]), ptr(t[1]), ptr(t[2]), ptr(t[3]), ptr(t[4]), ptr(t[5]), ptr(t[6]), ptr(o), ptr(po), ptr(pl), sm_scale, int(B), int(H),
                               int(c), int(dq - c), int(M), int(W), stream_of(q));
     if (rc != 0) return code(rc);
     if (a[11] != Py_None) { Py_INCREF(a[11]);  return a[11]; }
@@ -302,7 +315,7 @@ PyObject* rope_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!out.take(a[7], at::kBFloat16, {rows, vecs, c}, x)) return none();
     p.n_rows = rows;  p.vecs_per_row = int(vecs);  p.c = int(c);  p.n_rope = 64;  p.inverse = inverse;
     p.x = ptr(x);  p.out = ptr(out.t);  p.positions = ptr<int32_t>(pos);  p.norm_weight = ptr(w);
-    const int rc = lib.rope_norm(&p, stream_of(x));
+    const int rc = launch(lib.rope_norm, &p, stream_of(x));
     return rc != 0 ? code(rc) : out.result();
 }
 
@@ -326,7 +339,7 @@ PyObject* insert(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (rows->size(2) != kQk || !fits32(B) || !fits32(T) || !has_shape(n_rows, {B}) || !cache_dest(a[1], a[2], a[3], a[5], B, &d)) return none();
     Dsv4KvQuantizeInsertParams p{};
     p.B = int(B);  p.T = int(T);  p.rows = ptr(rows);  p.stride_b = T * kQk;  p.stride_t = kQk;  p.n_rows = ptr<int32_t>(n_rows);  p.dst = &d;
-    const int rc = lib.insert(&p, stream_of(rows));
+    const int rc = launch(lib.insert, &p, stream_of(rows));
     if (rc != 0) return code(rc);
     Py_RETURN_TRUE;
 }
@@ -352,7 +365,7 @@ PyObject* csa_compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.B = int(B);  p.n = int(rows);  p.c_out = int(c);  p.m = int(m);
     p.C_a = ptr(t[0]);  p.C_b = ptr(t[1]);  p.Z_a = ptr(t[2]);  p.Z_b = ptr(t[3]);  p.B_a = ptr(t[4]);  p.B_b = ptr(t[5]);  p.out = ptr(out.t);
     p.stride_C_b = rows * c;  p.stride_C_n = c;  p.stride_out_b = (rows / m) * c;  p.stride_out_blk = c;
-    const int rc = lib.csa_compress(&p, stream_of(t[0]));
+    const int rc = launch(lib.csa_compress, &p, stream_of(t[0]));
     return rc != 0 ? code(rc) : out.result();
 }
 
@@ -376,7 +389,7 @@ PyObject* hca_compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Dsv4HcaCompressParams p{};
     p.B = int(B);  p.n = int(rows);  p.c = int(c);  p.m = int(m);  p.C = ptr(C);  p.Z = ptr(Z);  p.bias = ptr(bias);
     p.stride_b = rows * c;  p.stride_n = c;  p.out = ptr(out.t);  p.dst = insert ? &d : nullptr;
-    const int rc = lib.hca_compress(&p, stream_of(C));
+    const int rc = launch(lib.hca_compress, &p, stream_of(C));
     if (rc != 0) return code(rc);
     if (with_out) return out.result();
     Py_RETURN_FALSE;
@@ -408,7 +421,7 @@ PyObject* indexer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.B = int(B);  p.s_q = int(s_q);  p.max_pages = int(pages);  p.k = int(k);  p.num_pages = keys->size(0);  p.score_stride = scores.t->size(1);
     p.q_fp8 = ptr(q);  p.q_weight = ptr<float>(w);  p.key_pages = ptr(keys);  p.block_table = ptr<int32_t>(table);  p.n_vis = ptr<int32_t>(vis);
     p.scores = ptr<float>(scores.t);  p.out_indices = ptr<int32_t>(out.t);  p.status = ptr<int32_t>(status);
-    const int rc = lib.indexer(&p, stream_of(q));
+    const int rc = launch(lib.indexer, &p, stream_of(q));
     return rc != 0 ? code(rc) : pair(out, scores);
 }
 
@@ -428,7 +441,7 @@ PyObject* plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.kind = int(v[0]);  p.B = int(v[1]);  p.s_q = int(v[2]);  p.H = int(v[3]);  p.topk = int(v[4]);  p.num_splits = int(v[5]);  p.num_sms = int(v[6]);
     p.topk_len = ptr<int32_t>(t[0]);  p.kv_len = ptr<int32_t>(t[1]);  p.win_len = ptr<int32_t>(t[2]);
     p.sched = ptr(t[3]);  p.sched_bytes = int64_t(t[3]->nbytes());
-    return code(lib.plan(&p, stream_of(t[3])));
+    return code(launch(lib.plan, &p, stream_of(t[3])));
 }
 
 // (partial_o, partial_lse, attn_sink, out, lse)
@@ -450,7 +463,7 @@ PyObject* combine(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.partial_o = ptr<float>(po);  p.partial_lse = ptr<float>(pl);  p.out = ptr(out.t);  p.lse = ptr<float>(lse.t);  p.attn_sink = ptr<float>(sink);
     p.stride_po_split = N * H * D;  p.stride_po_n = H * D;  p.stride_po_h = D;  p.stride_pl_split = N * H;  p.stride_pl_n = H;
     p.stride_out_n = H * D;  p.stride_out_h = D;  p.stride_lse_n = H;
-    const int rc = lib.combine(&p, stream_of(po));
+    const int rc = launch(lib.combine, &p, stream_of(po));
     return rc != 0 ? code(rc) : pair(out, lse);
 }
 
