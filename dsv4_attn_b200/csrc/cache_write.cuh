@@ -62,8 +62,8 @@ __device__ __forceinline__ float block_scale(float absmax) {
 // x / scale from the correctly rounded reciprocal r = RN(1 / scale): one multiply, the
 // remainder by FMA, one corrective FMA (Markstein's division step for machines with a fused multiply-add: P. Markstein,
 // IBM Journal of Research and Development 34(1), 1990).  Three instructions
-// instead of the dozen of a general division, whose range handling is not needed here: scale is
-// a normal number and |x / scale| <= 448.  The step reproduced the IEEE quotient on every one of
+// instead of the dozen of a general division, whose range handling is not needed here: scale is no smaller than 2^-100
+// (lift_small) and |x / scale| <= 448.  The step reproduced the IEEE quotient on every one of
 // 8e7 random (x, scale) pairs checked on the CPU; a last-bit difference could change the e4m3
 // byte only on an exact rounding boundary, and the GPU tests compare every byte written with
 // the CPU restatement's.
@@ -73,6 +73,17 @@ __device__ __forceinline__ float div_by_scale(float x, float scale, float r) {
     return fmaf(rem, r, q);
 }
 
+// A block so small that the reciprocal of its scale (infinite from 2^-128 down) or the division step's remainder would leave FP32's
+// range is divided 2^64 times as large by a divisor 2^64 times as large: the same quotients, and both products are exact.
+template <int N>
+__device__ __forceinline__ float lift_small(float (&f)[N], float scale) {
+    if (scale >= 0x1p-100f) return scale;
+#pragma unroll
+    for (int k = 0; k < N; ++k) f[k] *= 0x1p64f;
+    return scale * 0x1p64f;
+}
+
+// four values of a block over its (lifted) scale
 __device__ __forceinline__ uint32_t quant4(float a, float b, float c, float d, float scale) {
     const float r = __frcp_rn(scale);
     const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(div_by_scale(a, scale, r), div_by_scale(b, scale, r)), __NV_SATFINITE, __NV_E4M3);
@@ -263,9 +274,10 @@ __global__ void __launch_bounds__(kHcaCompressThreads, 2) hca_compress_kernel(co
         for (int d = 1; d < 16; d <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, d));
         const float scale = block_scale(amax);
         if (entry != nullptr) {
+            const float divisor = lift_small(o, scale);
             uint2 q;
-            q.x = quant4(o[0], o[1], o[2], o[3], scale);
-            q.y = quant4(o[4], o[5], o[6], o[7], scale);
+            q.x = quant4(o[0], o[1], o[2], o[3], divisor);
+            q.y = quant4(o[4], o[5], o[6], o[7], divisor);
             *reinterpret_cast<uint2*>(entry + t * 8) = q;
             if ((t & 15) == 0) *reinterpret_cast<float*>(entry + 512 + 4 * (t >> 4)) = scale;
         }
@@ -322,11 +334,12 @@ __global__ void __launch_bounds__(kInsertThreads) kv_quantize_insert_kernel(cons
         for (int d = 1; d < 8; d <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, d));
         const float scale = block_scale(amax);
         if (entry == nullptr) continue;
+        const float divisor = lift_small(f, scale);
         uint4 q;
-        q.x = quant4(f[0], f[1], f[2], f[3], scale);
-        q.y = quant4(f[4], f[5], f[6], f[7], scale);
-        q.z = quant4(f[8], f[9], f[10], f[11], scale);
-        q.w = quant4(f[12], f[13], f[14], f[15], scale);
+        q.x = quant4(f[0], f[1], f[2], f[3], divisor);
+        q.y = quant4(f[4], f[5], f[6], f[7], divisor);
+        q.z = quant4(f[8], f[9], f[10], f[11], divisor);
+        q.w = quant4(f[12], f[13], f[14], f[15], divisor);
         *reinterpret_cast<uint4*>(entry + 16 * lane) = q;
         if ((lane & 7) == 0) *reinterpret_cast<float*>(entry + 512 + 4 * (lane >> 3)) = scale;
         *reinterpret_cast<uint32_t*>(entry + 528 + 4 * lane) = rope;

@@ -216,3 +216,25 @@ def test_rope_norm_vs_reference_outputs(lib, name):
     assert (y[..., -64:].float() - dx[..., -64:].float()).abs().max().item() <= 4e-2
     with pytest.raises(ValueError):
         lib.rope_norm(dx[..., :100].contiguous(), dpos)
+
+
+def test_quantisers_bit_exact_on_tiny_rows(lib):
+    """Blocks so small that their scale is at the end of FP32's range or below its normal numbers: the reciprocal of the scale would be
+    infinite and the entry hold NaN bytes, for every later decode."""
+    rng = np.random.default_rng(66)
+    B, T = 1, 64
+    rows = rng.standard_normal((B, T, 576)).astype(np.float32)
+    rows = orc.bf16_round(rows * np.float32(2.0) ** -np.linspace(60, 132, T).round().astype(np.float32)[None, :, None])
+    rows += np.float32(0)                                      # (-0 becomes 0, as in the compressor's sum)
+    pool, bt = make_pool(rng, B, 1)
+    pos = np.zeros(B, np.int32)
+    want = orc.quantize_insert(pool, bt, pos, rows)
+    assert not (want[bt[0, 0], :, :512] & 0x7F == 0x7F).any()
+    got = gu.dev(pool)
+    lib.kv_quantize_insert(bf(rows), got, gu.dev(bt), gu.dev(pos))
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
+    # the compressor's fused insert: blocks of one row come out as they went in
+    got = gu.dev(pool)
+    lib.hca_compress_fwd(bf(rows), bf(np.zeros_like(rows)), bf(np.zeros((1, 576), np.float32)), 1, kv_pool=got, block_table=gu.dev(bt),
+                         insert_pos=gu.dev(pos), want_out=False)
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
