@@ -57,11 +57,10 @@ __device__ __forceinline__ void merge_head(const CombineArgs& a, int n, int h, i
     float mx = l_first;
     for (int s = lane + 32; s < S; s += 32) mx = fmaxf(mx, ptx::ld(pl + int64_t(s) * pl_stride));
     mx = warp_max(mx);
-    float sum = 0.f;
-    if (mx != -CUDART_INF_F) {
-        sum = exp2f(l_first - mx);
-        for (int s = lane + 32; s < S; s += 32) sum += exp2f(ptx::ld(pl + int64_t(s) * pl_stride) - mx);
-    }
+    // (the maximum leaves NaN out; the sum does not, whether all splits are NaN or some)
+    const float ref = (mx == -CUDART_INF_F) ? 0.f : mx;
+    float sum = exp2f(l_first - ref);
+    for (int s = lane + 32; s < S; s += 32) sum += exp2f(ptx::ld(pl + int64_t(s) * pl_stride) - ref);
     sum = warp_sum(sum);
     const bool has = sum != 0.f;
     const float glse = has ? log2f(sum) + mx : -CUDART_INF_F;

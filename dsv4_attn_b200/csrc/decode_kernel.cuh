@@ -1374,9 +1374,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
             float denom = l_sum;
             if (final_out && a.attn_sink != nullptr && write) {
                 const float s2 = ptx::ld(a.attn_sink + h0 + r) * 1.4426950408889634f;
-                denom = (l_sum > 0.f) ? l_sum + ptx::ex2(s2 - m_ref) : 1.f;   // empty row: O is 0 anyway
+                denom = (l_sum != 0.f) ? l_sum + ptx::ex2(s2 - m_ref) : 1.f;   // empty row: O is 0 anyway
             }
-            const float inv = (l_sum > 0.f) ? 1.f / denom : 0.f;
+            const float inv = (l_sum != 0.f) ? 1.f / denom : 0.f;
             // O leaves through shared memory: each thread owns half a row in tensor memory, but rows are 1 KB apart in global
             // memory, so 64 columns at a time are laid down in this warp's own 64 bytes per row of each P buffer (swizzled like
             // P; the MMAs that read P have completed, and the next P there is written by this warp) and written
@@ -1412,9 +1412,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
                 __syncwarp();
             }
             if (write && colhalf == 0) {
-                const float lse2 = (l_sum > 0.f) ? m_ref + log2f(l_sum) : -CUDART_INF_F;
+                const float lse2 = (l_sum != 0.f) ? m_ref + log2f(l_sum) : -CUDART_INF_F;
                 if (!final_out) a.partial_lse[prow0 + r] = lse2;
-                else if (a.lse != nullptr) a.lse[int64_t(n) * a.H + h0 + r] = (l_sum > 0.f) ? lse2 * 0.6931471805599453f : -CUDART_INF_F;
+                else if (a.lse != nullptr) a.lse[int64_t(n) * a.H + h0 + r] = (l_sum != 0.f) ? lse2 * 0.6931471805599453f : -CUDART_INF_F;
             }
         }
     }

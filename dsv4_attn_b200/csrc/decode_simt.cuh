@@ -143,13 +143,13 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeA
         for (int i = 0; i < 4; ++i) acc[i] = fmaf(p, row_value<SRC>(r, tid * 4 + i), acc[i]);
     }
     float denom = lsum;
-    if (a.attn_sink != nullptr && lsum > 0.f) denom += exp2f(a.attn_sink[h] * 1.4426950408889634f - lmax);
-    const float inv = lsum > 0.f ? 1.f / denom : 0.f;
+    if (a.attn_sink != nullptr && lsum != 0.f) denom += exp2f(a.attn_sink[h] * 1.4426950408889634f - lmax);
+    const float inv = lsum != 0.f ? 1.f / denom : 0.f;
     __nv_bfloat16* o = a.out + (int64_t(n) * a.H + h) * 512 + tid * 4;
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[i] = __float2bfloat16_rn(acc[i] * inv);
     if (tid == 0 && a.lse != nullptr)
-        a.lse[int64_t(n) * a.H + h] = lsum > 0.f ? (lmax + log2f(lsum)) * 0.6931471805599453f : -CUDART_INF_F;
+        a.lse[int64_t(n) * a.H + h] = lsum != 0.f ? (lmax + log2f(lsum)) * 0.6931471805599453f : -CUDART_INF_F;
 }
 
 }  // namespace dsv4

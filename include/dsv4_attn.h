@@ -64,6 +64,8 @@ extern "C" {
  * scales <= 146 - a block with a larger scale (entries beyond +-65408) is clamped to 146.  Inputs
  * of the N(0,1) kind the cache is built for are far inside both; dsv4_attn_b200.api offers a
  * host-side check (check_fp16_range=True) for callers that cannot vouch for theirs.
+ * A query row (one token, one head) that is NaN, or leaves that range, gives NaN in its own row of out
+ * and lse, with or without splits, and nowhere else (all decode entry points).
  */
 typedef struct Dsv4CsaSparseDecodeParams {
     int32_t B;                  /* requests */

@@ -81,3 +81,6 @@ def test_nonfinite_queries_spoil_their_own_rows_only(lib, source, route, H, n, v
         gu.check_out(gu.out_to_f32(out).reshape(B, H, -1)[keep], want.reshape(B, H, -1)[keep], what)
         if lse is not None:
             gu.check_lse(lse.cpu().numpy().reshape(B, H)[keep], want_lse.reshape(B, H)[keep], what)
+        # the spoilt rows say so, in splits and pieces as well (-inf would read as an empty row)
+        assert np.isnan(gu.out_to_f32(out).reshape(B, H, -1)[~keep]).all(), what
+        assert lse is None or np.isnan(lse.cpu().numpy().reshape(B, H)[~keep]).all(), what
