@@ -40,27 +40,18 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
     }
 }
 
-// Vector of VEC BF16 values and its FP32 unpacking: 16-byte vectors for VEC = 8, 8-byte for VEC = 4.
-template <int VEC> struct BfVec;
-template <> struct BfVec<8> {
-    using T = uint4;
-    static __device__ __forceinline__ T load_stream(const __nv_bfloat16* p) { return ptx::ldg_stream_v4(p); }
-    static __device__ __forceinline__ void unpack(const T& v, float (&f)[8]) { unpack8(v, f); }
-};
-template <> struct BfVec<4> {
-    using T = uint2;
-    static __device__ __forceinline__ T load_stream(const __nv_bfloat16* p) {
-        T v;
-        asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-        return v;
-    }
-    static __device__ __forceinline__ void unpack(const T& v, float (&f)[4]) {
-        f[0] = __uint_as_float(v.x << 16);  f[1] = __uint_as_float(v.x & 0xFFFF0000u);
-        f[2] = __uint_as_float(v.y << 16);  f[3] = __uint_as_float(v.y & 0xFFFF0000u);
-    }
-};
+// Four BF16 values and their FP32 unpacking.
+__device__ __forceinline__ uint2 load_stream4(const __nv_bfloat16* p) {
+    uint2 v;
+    asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void unpack4(const uint2& v, float (&f)[4]) {
+    f[0] = __uint_as_float(v.x << 16);  f[1] = __uint_as_float(v.x & 0xFFFF0000u);
+    f[2] = __uint_as_float(v.y << 16);  f[3] = __uint_as_float(v.y & 0xFFFF0000u);
+}
 
-// VEC = 8 / 4: 16- / 8-byte vectors (c_out % VEC == 0 and rows aligned to the vector); VEC = 1: any c_out.
+// VEC = 4: 8-byte vectors (c_out % 4 == 0 and rows aligned to the vector); VEC = 1: any c_out.
 template <int M, int VEC>
 __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_reduce_kernel(const CompressReduceArgs a) {
     ptx::pdl_trigger();
@@ -77,22 +68,22 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
         const int64_t row_a = int64_t(b) * a.stride_c_b + int64_t(blk) * M * a.stride_c_n + ch;
         const int64_t row_b = row_a - int64_t(M) * a.stride_c_n;      // previous block (blk > 0 only)
         float o[VEC];
-        if constexpr (VEC >= 4) {
-            using V = typename BfVec<VEC>::T;
+        if constexpr (VEC == 4) {
+            using V = uint2;
             // all 4m data vectors in flight first; the biases are small and cached, they are
             // re-read where needed so that the raw data can stay in registers
             V za[M], ca[M], zb[M], cb[M];
 #pragma unroll
             for (int j = 0; j < M; ++j) {
-                za[j] = BfVec<VEC>::load_stream(a.Z_a + row_a + j * a.stride_c_n);
-                ca[j] = BfVec<VEC>::load_stream(a.C_a + row_a + j * a.stride_c_n);
+                za[j] = load_stream4(a.Z_a + row_a + j * a.stride_c_n);
+                ca[j] = load_stream4(a.C_a + row_a + j * a.stride_c_n);
             }
             const bool has_b = blk > 0;
             if (has_b) {
 #pragma unroll
                 for (int j = 0; j < M; ++j) {
-                    zb[j] = BfVec<VEC>::load_stream(a.Z_b + row_b + j * a.stride_c_n);
-                    cb[j] = BfVec<VEC>::load_stream(a.C_b + row_b + j * a.stride_c_n);
+                    zb[j] = load_stream4(a.Z_b + row_b + j * a.stride_c_n);
+                    cb[j] = load_stream4(a.C_b + row_b + j * a.stride_c_n);
                 }
             }
             auto bias = [&](int j, bool bside) { return ptx::ld(reinterpret_cast<const V*>((bside ? a.B_b : a.B_a) + int64_t(j) * a.c_out + ch)); };
@@ -135,9 +126,9 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
 #pragma unroll
                     for (int j = 0; j < M; ++j) {
                         float z[VEC], u[VEC], c[VEC];
-                        BfVec<VEC>::unpack(side ? zb[j] : za[j], z);
-                        BfVec<VEC>::unpack(bias(j, side == 1), u);
-                        BfVec<VEC>::unpack(side ? cb[j] : ca[j], c);
+                        unpack4(side ? zb[j] : za[j], z);
+                        unpack4(bias(j, side == 1), u);
+                        unpack4(side ? cb[j] : ca[j], c);
 #pragma unroll
                         for (int k = 0; k < P; ++k) {
                             const uint64_t t = ptx::add_f32x2(ptx::pack_f32x2(z[2 * k], z[2 * k + 1]), ptx::pack_f32x2(u[2 * k], u[2 * k + 1]));
@@ -169,9 +160,9 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
 #pragma unroll
                         for (int j = 0; j < M; ++j) {
                             float z[VEC], u[VEC], c[VEC];
-                            BfVec<VEC>::unpack(side ? zb[j] : za[j], z);
-                            BfVec<VEC>::unpack(bias(j, side == 1), u);
-                            BfVec<VEC>::unpack(side ? cb[j] : ca[j], c);
+                            unpack4(side ? zb[j] : za[j], z);
+                            unpack4(bias(j, side == 1), u);
+                            unpack4(side ? cb[j] : ca[j], c);
 #pragma unroll
                             for (int k = 0; k < VEC; ++k) {
                                 if (pass == 0) {
@@ -219,12 +210,7 @@ __global__ void __launch_bounds__(kCompressThreads, VEC == 4 ? 3 : 2) compress_r
             o[0] = acc / sum;
         }
         __nv_bfloat16* dst = a.out + int64_t(b) * a.stride_out_b + int64_t(blk) * a.stride_out_blk + ch;
-        if constexpr (VEC == 8) {
-            uint4 w;
-            w.x = ptx::pack_bf16x2(o[0], o[1]);  w.y = ptx::pack_bf16x2(o[2], o[3]);
-            w.z = ptx::pack_bf16x2(o[4], o[5]);  w.w = ptx::pack_bf16x2(o[6], o[7]);
-            *reinterpret_cast<uint4*>(dst) = w;
-        } else if constexpr (VEC == 4) {
+        if constexpr (VEC == 4) {
             uint2 w;
             w.x = ptx::pack_bf16x2(o[0], o[1]);  w.y = ptx::pack_bf16x2(o[2], o[3]);
             *reinterpret_cast<uint2*>(dst) = w;

@@ -30,13 +30,12 @@ constexpr int kPlanFixedCost = 48;     // set-up and write-out of an item that t
 constexpr int kPlanMergeCost = 96;     // what cutting units costs a pair in partial traffic and merge time
 
 struct PlanArgs {
-    int kind;                    // SourceKind: where the lengths come from
+    int kind;                    // kSrcCsa or kSrcHca: where the lengths come from
     int rows, hgs;               // rows = B * s_q, hgs = groups of 128 heads
     int topk;                    // CSA
     const int32_t* topk_len;     // CSA, optional
-    const int32_t* kv_len;       // CSA optional (passed through), HCA / packed pages required
-    const int32_t* win_len;      // HCA / packed pages
-    int ref_m_cur, ref_swa_len;  // reference planes
+    const int32_t* kv_len;       // CSA optional (passed through), HCA required
+    const int32_t* win_len;      // HCA
     int num_pairs;
     int fixed_splits;            // 0: balance over the pairs; >= 1: that many equal pieces per unit
     int item_cap, slot_cap;
@@ -53,12 +52,9 @@ __host__ __device__ __forceinline__ void plan_row_lengths(const PlanArgs& p, int
         const int raw = (p.topk_len != nullptr) ? p.topk_len[row] : p.topk;
         n_tok = raw < 0 ? 0 : (raw > p.topk ? p.topk : raw);
         kv_len_n = (p.kv_len != nullptr) ? p.kv_len[row] : 0x7FFFFFFF;
-    } else if (p.kind == kSrcHca || p.kind == kSrcRefPaged) {
+    } else {
         kv_len_n = p.kv_len[row] > 0 ? p.kv_len[row] : 0;
         n_tok = kv_len_n + (p.win_len[row] > 0 ? p.win_len[row] : 0);
-    } else {
-        kv_len_n = p.ref_m_cur;
-        n_tok = p.ref_m_cur + p.ref_swa_len;
     }
 }
 
