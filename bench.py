@@ -83,10 +83,10 @@ DEFAULT_WORKLOAD = "hca_b64_h128_ctx100k"
 # DRAM bytes (read + write) of ONE launch of the decode kernel on the workload, from an ncu
 # capture of that launch (dram__bytes_read.sum + dram__bytes_write.sum); the summaries
 # under profiles/ hold the figures and the command lines.
-NCU_DRAM_TRAFFIC = {"hca_b64_h128_ctx100k": 47.79e6, "csa_b64_h128_topk512_ctx3072": 32.43e6,
-                    # captured on the B = 16 slice of the same shape (27.51 MB per launch) and scaled by the rows
-                    "csa_b64_h128_topk2048_ctx100k": 4 * 27.51e6}
-NCU_TRAFFIC_SOURCE = "ncu capture of one launch (profiles/decode_mma_kernel_*.md)"
+NCU_DRAM_TRAFFIC = {"hca_b64_h128_ctx100k": 47.85e6, "csa_b64_h128_topk512_ctx3072": 33.08e6,
+                    # captured on the B = 16 slice of the same shape (29.39 MB per launch) and scaled by the rows
+                    "csa_b64_h128_topk2048_ctx100k": 4 * 29.39e6}
+NCU_TRAFFIC_SOURCE = "ncu capture of one launch (profiles/decode_mma_kernel_counters.md)"
 
 
 def measured_peak_gbs():
@@ -112,7 +112,7 @@ def tensor_view(kv_bytes, H, ms):
     src = "measured" if peak else "fallback"
     peak = peak or 1590.0
     return {"bound": "tensor", "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak, "peak_source": src,
-            "note": "useful FLOPs only; each block also recomputes QK for the other half of the value columns"}
+            "note": "useful FLOPs only"}
 
 
 # ───────────────────────── clocks sampling ─────────────────────────

@@ -570,8 +570,12 @@ extern "C" int dsv4_attn_plan_splits(int rows, int H, int max_len, int num_sms) 
     // Cost model in units of one tile's time: a block costs a fixed set-up (Q
     // load, tensor-memory allocation, epilogue) plus its tiles; blocks run in
     // waves of `num_sms`; splitting adds the partial write + merge read, and the merge of one row takes its splits in turn.
-    // constants fitted to measurements on B200 (split sweeps, 1 to 100 rows x 2 to 64 tiles: within 4 % of the best split count;
-    // a set-up of 4 tiles cut 48 rows of 32 tiles in three, 59 us against 55, and one such row in 32, 23 us against 19)
+    // Constants fitted to 656-byte CSA rows of 128 heads on B200 (1.3 us a tile, 11 us a launch).  1 to 100 rows x 2 to 32 tiles, every split
+    // count: within 1 % of the best one at 39 of 48 shapes and within 7 % at 46; the exceptions are 4 and 8 rows of four tiles, which stay whole (15.0 us)
+    // where four splits take 12.6.  The reference layouts, at 1.7 to 2.2 us a tile, go by the same constants: packed pages 1 to
+    // 100 rows x 4 to 32 tiles within 7 % at 37 of 40 shapes, four-tile rows up to 28 % above the best (17.0 against 13.3 us).  Their length is the block tables' capacity, which is what the
+    // host knows; rows much shorter than that may be cut more often than they need.
+    // (A set-up of 4 tiles cut 48 rows of 32 tiles in three, 59 us against 55, and one such row in 32, 23 us against 19.)
     const double fixed = 7.0, merge_per_split = 1.8, merge_launch = 2.0, merge_serial = 0.2;
     double best = 1e300;
     int best_s = 1;

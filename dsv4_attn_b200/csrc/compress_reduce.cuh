@@ -6,7 +6,8 @@
 // thread then holds 16 vectors = 32 registers of raw data).  Bound by HBM and, close behind, by instruction issue: the
 // arithmetic is done two channels at a time (packed BF16 for the reference maximum, packed FP32 for the rest), 230
 // instructions a thread instead of 420, and three blocks fit an SM at 80 registers (at four and 64 registers it
-// spills: 34 us).  32k rows: 34 -> 30 us, 5.0 TB/s.  The grid is sized so that all SMs hold two waves
+// spills).  32k rows of 576, back to back on rotating inputs: 30.8 -> 28.5 us, 5.6 TB/s (28.1 without the bound on
+// the reference maximum below).  The grid is sized so that all SMs hold two waves
 // of resident blocks.
 #pragma once
 

@@ -23,15 +23,16 @@
 //                  reference maximum, write P to shared memory, rescale O in tensor memory when the maximum
 //                  moved, and finally normalise and store.
 //
-// What bounds it, in SM cycles per tile: tensor pipe 24 x 18 + 12 x 25 (S) + 8 x 64 (O) = 1244; shared-memory port
-// (128 B/clk) about 2000: raw records in and out 520, operand writes 610, operand reads 860; TMA gather of 656-byte records
-// 1200 alone, up to 1900 with every SM gathering from DRAM.  Loads through the load/store unit (4 records x 128 bytes per
-// instruction, straight into registers) took 3300 cycles a tile: records at a pitch of 656 bytes cost eight tag
-// look-ups per instruction.  Measured, B200, 128 heads: CSA, 64 requests x top-k 2048 59 us (one block per SM with its own copy of
-// S: 92), HCA, 64 requests x 910 entries 32 us (45): 1.45-1.6 us a tile (2.0-2.9) and some 11 us a launch.
+// What bounds it, in SM cycles per tile: tensor pipe 24 x 18 + 12 x 25 (S) + 8 x 64 (O) = 1244 (counted: 1445); shared-memory port
+// (128 B/clk) about 2000 (counted: bank reads 1172 + writes 845 = 2017): raw records in and out 520, operand writes 610, operand reads 860;
+// TMA gather of 656-byte records 1200 alone, up to 1900 with every SM gathering from DRAM.  A tile takes 2380 with few SMs at work, 2570 with
+// all of them and the inputs in L2, 2630 from DRAM: the port is busy for 77 to 85 % of it.  Loads through the load/store unit (4 records
+// x 128 bytes per instruction, straight into registers) took 3300: records at a pitch of 656 bytes cost eight tag look-ups per
+// instruction.  Measured, B200, 128 heads, inputs from DRAM: CSA, 64 requests x top-k 2048 60 us (one block per SM with its own copy of
+// S: 92), HCA, 64 requests x 910 entries 32 us (45): 1.34 us a tile (2.0-2.9) and some 12 us a launch.
 //
 // All waits are bounded; a wait that gives up records where in `status` and the pair leaves through the common
-// exit, freeing its tensor memory.
+// exit, where it stays until its copies and MMAs in flight have landed, and frees its tensor memory.
 #pragma once
 
 #include <cuda.h>
@@ -774,8 +775,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1) deco
         else ptx::mbar_arrive_remote(ptx::mapa(bar, 0));
     };
 
-    // On the static grid a packed-layout launch sees to Q before anything is known of the row.  (The reference planes, with no lengths,
-    // indices or tables to wait for, have their first records before Q: 1 us of 45 slower with Q first.)
+    // On the static grid a launch over 656-byte records sees to Q before anything is known of the row (top-k 2048, 64 requests: 62.5 -> 60.3 us).
+    // The reference planes, with no lengths, indices or tables to wait for, have their first records before Q: 1 us of 45 slower with Q first.
+    // Packed reference pages (40 ragged requests): 48.0 to 48.3 us either way.  On a schedule Q comes item by item; its first one early was not tried.
     const bool early_q = use_f16(SRC) && !sched;
 
     // ── set-up ──

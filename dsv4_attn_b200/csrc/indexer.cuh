@@ -12,9 +12,10 @@
 //    memory lane = key, columns = (token, head).  Warp roles: one TMA producer
 //    lane, one MMA-issuing lane, four epilogue warps; a ring of key stages and two
 //    accumulator buffers in tensor memory decouple the three.
-//  * topk_select_kernel: per (request, token) row a radix select over the FP32
-//    scores (four 8-bit rounds, histograms in shared memory), then a compaction
-//    pass that writes the indices of the k best (unordered; -1 padded).
+//  * topk_select_kernel / topk_select_pair_kernel: per (request, token) row a histogram over
+//    1024 equal-width value bins finds the bin of the k-th largest score; higher bins are
+//    selected whole, the entries of that bin by comparison (or an exact radix select when
+//    there are many).  Writes the indices of the k best (unordered; -1 padded).
 //
 // Key page: 64 keys x 128 e4m3 bytes, then the 64 FP32 scales of those keys
 // (8448 bytes = 66 rows of 128 bytes).

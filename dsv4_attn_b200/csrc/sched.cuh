@@ -154,7 +154,8 @@ __device__ __forceinline__ T plan_block_scan(T v, T* warp_sums) {
 
 // One block: the time is the chain of its steps (load, scan, deal, scan, write), not bandwidth.  A thread keeps the lengths, cost and
 // prefix of its first unit in registers from pass to pass (all there are up to 1024 units), both sums are block scans, and
-// the divisions are 32-bit where they can be: 256 rows take xx us (9.3 with one thread adding up the pairs and everything read back from memory).
+// the divisions are 32-bit where they can be.  Back to back in a graph, 64 / 256 / 1024 rows: 7.2 / 6.1 / 8.5 us (8.5 / 7.6 / 9.7 with one thread adding up the
+// pairs and everything read back from memory); launched alone after an L2 flush 12 to 19 us, most of it the launch.
 __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const __grid_constant__ PlanArgs p) {
     __shared__ long long s_warp[32];
     __shared__ int s_warp_i[32];
