@@ -162,8 +162,8 @@ def test_plan_for_another_batch_is_rejected(lib):
 @pytest.mark.parametrize("B,k", [(2, 512), (30, 2048), (40, 512), (60, 2048)])
 def test_plan_and_decode_back_to_back(lib, B, k):
     """The decode kernel is launched while the planner may still run: what it reads of the plan has to be the new one.  The schedule's
-    memory holds another plan when the planner starts, and nothing comes between planner and decode; 60 rows take the merge that shares out
-    the cut units, the others the one that looks every row up."""
+    memory holds another plan when the planner starts, and nothing comes between planner and decode; 40 and 60 rows take the merge that
+    shares out the cut units, the others the one that looks every row up."""
     case = orc.make_csa_case(seed=400 + B, B=B, s_q=1, H=128, n_entries=k + 64, topk=k)
     args = gu.csa_to_dev(case)
     want, want_lse = lib.csa_sparse_decode(**args, num_splits=1)
